@@ -244,7 +244,7 @@ def prepare(case, seed):
             st["seed"] = seed
     elif c["kind"] == "eprop":
         g = _ff_graph(c, seed) if c["net"] == "ff" else _audio_graph(c, seed)
-        cfg = eprop.TrainConfig(lif=st["lif"], lr=0.02, trace_decay=0.95, mode=MODES[c["mode"]], seed=seed)
+        cfg = eprop.TrainConfig(lif=st["lif"], lr=5e-4, trace_decay=0.95, mode=MODES[c["mode"]], seed=seed)
         st["session"] = eprop.create(g, cfg, c["samples"], weights=g.weights)
         st["events"], st["steps"] = _events(c, seed, c["n_in"])
         if not c["update"]:
