@@ -105,7 +105,8 @@ void free_graph(Graph* g) {
   for (void* p : {(void*)g->row_ptr, (void*)g->edges, (void*)g->post, (void*)g->col_of,
                   (void*)g->out_ch, (void*)g->role, (void*)g->channel, (void*)g->colbase,
                   (void*)g->gedges, (void*)g->gptr, (void*)g->groups, (void*)g->ibase,
-                  (void*)g->chan_ptr, (void*)g->chan_ids, (void*)g->ro_rank, (void*)g->ro_chan})
+                  (void*)g->chan_ptr, (void*)g->chan_ids, (void*)g->ro_rank, (void*)g->ro_chan,
+                  (void*)g->sedges, (void*)g->sptr, (void*)g->crange})
     dev_free(p);
 }
 
@@ -213,6 +214,26 @@ int setup_tables(Graph* g, int n, int m, int max_delay, const int32_t* row_ptr,
     const long long lg = (long long)std::log2(std::max(1, n)) * 64 + (long long)std::log2(std::max(1, m));
     g->signature = (lg << 16) ^ ((long long)(g->fanin_cv * 4) << 8) ^ (long long)g->R;
   }
+  // column ranges of about equal in-degree for the sample-per-CTA kernel: the
+  // columns by descending in-degree, each to the range with the least so far
+  // (first of equals), so hub columns spread over the ranges
+  std::vector<uint8_t> crange;
+  if (tier_s_possible(g)) {
+    crange.resize((size_t)std::max(1, nc));
+    std::vector<int> ids;
+    ids.reserve((size_t)nc);
+    for (int i = 0; i < n; ++i)
+      if (indeg[i] > 0) ids.push_back(i);
+    std::stable_sort(ids.begin(), ids.end(), [&](int x, int y) { return indeg[x] > indeg[y]; });
+    long long load[kSRanges] = {};
+    for (int i : ids) {
+      int r = 0;
+      for (int k = 1; k < kSRanges; ++k)
+        if (load[k] < load[r]) r = k;
+      crange[g->col_of_h[i]] = (uint8_t)r;
+      load[r] += indeg[i];
+    }
+  }
   std::vector<uint8_t> role(role_v, role_v + n);
   std::vector<int> channel(channel_v, channel_v + n);
   // leaky readout units: the OUTPUT neurons with a channel, ascending id
@@ -226,6 +247,7 @@ int setup_tables(Graph* g, int n, int m, int max_delay, const int32_t* row_ptr,
   int rc;
   if ((rc = dev_upload(&g->col_of, g->col_of_h.data(), (size_t)n))) return rc;
   if ((rc = dev_upload(&g->out_ch, out_ch.data(), (size_t)n))) return rc;
+  if (!crange.empty() && (rc = dev_upload(&g->crange, crange.data(), crange.size()))) return rc;
   if ((rc = dev_upload(&g->role, role.data(), role.size()))) return rc;
   if ((rc = dev_upload(&g->channel, channel.data(), channel.size()))) return rc;
   if ((rc = dev_upload(&g->colbase, colbase.data(), colbase.size()))) return rc;

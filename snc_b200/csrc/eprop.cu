@@ -50,11 +50,12 @@ struct snc_b200_eprop {
   int2* cin = nullptr;            // [S]
   int* gptr = nullptr;            // [ncols + 1]
   int n_groups = 0;
-  // grid mode: one sample's state does not fit one CTA's shared memory, so
-  // the forward runs on the all-SM kernel, which reads destination-grouped
-  // edges: a grouped copy of the trainer's weights, kept in step with them
+  // the forward kernels read regrouped edges: a regrouped copy of the
+  // trainer's weights, kept in step with them -- by column range for the
+  // sample-per-CTA kernel, by destination block in grid mode (one sample's
+  // state does not fit one CTA's shared memory: the all-SM kernel)
   bool grid = false;
-  int* gperm = nullptr;           // [S] CSR edge -> its grouped position
+  int* gperm = nullptr;           // [S] CSR edge -> its regrouped position
   uint2* gedges = nullptr;        // [S+2]
   sncb::Run* run = nullptr;
 };
@@ -127,14 +128,14 @@ __global__ void k_get_weights(int S, const uint2* edges, float* w) {
 
 static inline int grid_of(long long n, int b = 256) { return (int)std::max(1ll, (n + b - 1) / b); }
 
-// The grouped copy of the trainer's weights follows the CSR edges.
+// The regrouped copy of the trainer's weights follows the CSR edges.
 __global__ void k_sync_gedges(int S, const uint2* edges, const int* gperm, uint2* gedges) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < S) gedges[gperm[e]].y = edges[e].y;
 }
 
 static int sync_gedges(snc_b200_eprop* s, cudaStream_t st) {
-  if (!s->grid || s->g->S == 0) return SNC_B200_OK;
+  if (s->g->S == 0) return SNC_B200_OK;
   k_sync_gedges<<<grid_of(s->g->S), 256, 0, st>>>(s->g->S, s->edges, s->gperm, s->gedges);
   SNCB_CUDA(cudaGetLastError());
   return SNC_B200_OK;
@@ -315,7 +316,12 @@ static int create_session(snc_b200_eprop* s, const Graph* g, const snc_lif* lif,
     const int mode = cfg->mode == SNC_B200_MODE_SORT ? SNC_B200_MODE_SORT : SNC_B200_MODE_ATOMIC;
     s->grid = tier_s_smem_bytes(g, mode, true) > optin;
   }
-  if (s->grid) {
+  if (!s->grid) {
+    if ((rc = dev_alloc(&s->gperm, (size_t)S))) return rc;
+    if ((rc = dev_alloc(&s->gedges, (size_t)S + 2))) return rc;
+    if ((rc = regroup_by_range(g, s->edges, s->gedges, nullptr, s->gperm))) return rc;
+    SNCB_CUDA(cudaDeviceSynchronize());
+  } else {
     // the stable regroup of every row by destination block, as the graph's
     // grouped edges were built
     std::vector<int> post((size_t)std::max(1, S));
@@ -443,6 +449,7 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
     e.g = g;
     e.in = &in;
     e.edges = s->edges;
+    e.sedges = s->gedges;
     e.counts = s->counts;
     e.spikes = s->spikes;
     e.events = s->events;

@@ -99,8 +99,13 @@ struct FwdArgs {
   float* elig;
   unsigned long long* fires;
   float gamma, trace_decay;
-  int s_table;  // tier S SORT: 1 the whole-chunk cell table, 2 also the cell bitmaps
-  int s_lean;   // tier S SORT with the table: the column-list arrays left out
+  // tier S: edges with each row regrouped by column range, (delay * ncols +
+  // column, weight), and the segment starts [N][kSPtr]; fired rows whose
+  // segment starts shared memory holds at once; mask of the conflict tags
+  const uint2* sedges;
+  const int* sptr;
+  int s_cap;
+  int s_tmask;
   // deferred eligibility: psi of every ring column and step, [B][ncols][psi_T]
   // (null: eligibility accumulated in the forward into elig)
   float* psi_hist;
@@ -127,25 +132,12 @@ struct FwdArgs {
   int scan_only;
 };
 
-// Shared-memory bytes of the tier-S kernel for this graph.
-// Tier S SORT may add a per-cell table for whole chunks: kSTable keys, as
-// many list heads and one link per staged event.
-constexpr int kSTable = 2048;
-
-// With table == 2 four bitmaps of the ring's cells follow (two alternating
-// pairs: seen, hit more than once).
-static size_t cell_bitmap_words(int ncols, int R) { return ((size_t)R * ncols + 31) / 32; }
-
-static size_t tier_s_bytes(int N, int ncols, int R, int noc, int mode, bool eprop, int nthr,
-                           int table = 0, bool lean = false) {
+// Shared memory that decides whether a sample's state fits one CTA (tier S).
+// The kernel itself never needs more (tier_s_layout below).
+static size_t tier_s_bytes(int N, int ncols, int R, int noc, int mode, bool eprop, int nthr) {
   size_t words = (size_t)R * ncols + 4 * (size_t)N + (size_t)noc;
-  // SORT: row prefix, then the column-list arrays (head, tail, staged column,
-  // slot, weight, link) or, lean, the staged weights alone
-  if (mode == MODE_SORT)
-    words += (size_t)N + 1 + (table && lean ? (size_t)nthr : 2 * (size_t)ncols + 4 * (size_t)nthr);
+  if (mode == MODE_SORT) words += (size_t)N + 1 + 2 * (size_t)ncols + 4 * (size_t)nthr;
   if (eprop) words += (size_t)N + ncols;
-  if (mode == MODE_SORT && table) words += 2 * (size_t)kSTable + nthr;
-  if (mode == MODE_SORT && table == 2) words += 4 * cell_bitmap_words(ncols, R);
   return words * 4 + 16;
 }
 
@@ -218,12 +210,10 @@ __device__ __forceinline__ void apply_one(float* ring, int ring_stride, int col0
   }
 }
 
-// Chunks up to kCountMax events take the per-cell apply; above it tier S
-// uses unordered lists that every column sorts on its own, while tier G links
-// in order (its post blocks own hub columns whose per-step event count can be
-// large).
+// Chunks up to kCountMax events take the per-cell apply; larger ones are
+// linked in order (a post block owns hub columns whose per-step event count can
+// be large).
 constexpr int kCountMax = 256;
-constexpr int kRegSort = 16;
 constexpr int kFirstFlag = 1 << 30;  // marks a group's first event of its column in st_col
 
 // Ordered apply of a small chunk (ce <= kCountMax <= blockDim.x, so thread q
@@ -243,13 +233,13 @@ static_assert(kCellTable + kCountMax <= kGChunk, "the links live in st_col beyon
 
 // Table sizes (keys; as many list heads follow) and their hash bits.
 template <int TS>
-constexpr int kTabBits = TS == 2048 ? 11 : (TS == 1024 ? 10 : 9);
+constexpr int kTabBits = TS == 1024 ? 10 : 9;
 
 // Enters staged event q of cell (c, sl) into a table of TS keys (at most TS / 2
 // distinct cells); returns its entry.
 template <int TS>
 __device__ __forceinline__ unsigned cell_insert(int* tab, int* link, int q, int c, int sl, bool* first) {
-  static_assert(TS == 512 || TS == 1024 || TS == 2048, "table size");
+  static_assert(TS == 512 || TS == 1024, "table size");
   unsigned* key = reinterpret_cast<unsigned*>(tab);
   const unsigned k = (unsigned)c * 256u + (unsigned)sl + 1u;  // slot < 256, 0 = empty
   unsigned h = (k * 2654435761u) >> (32 - kTabBits<TS>);
@@ -348,67 +338,19 @@ __device__ void apply_cells(int ce, int* tab, int* st_col, const int* st_slot, c
 // block-local column st_col[q] (head / tail of every local column = -1).
 // Every ring cell must receive its contributions in increasing q.
 //  - chunks up to kCountMax events: apply_cells (above);
-//  - chunks up to serial_max: every warp links the events of its 32-event groups
+//  - larger chunks: every warp links the events of its 32-event groups
 //    (match.any: successor within the group, first event of each column
 //    flagged), then one warp joins the groups in staging order through the
 //    column tails -- one shared-memory round trip per group; one thread per
 //    column then replays its list: O(events), no sorting, and hub columns
 //    with many events in one step stay linear.
-//  - large chunks: lists are built in parallel with atomicExch (arbitrary
-//    order); each column thread loads up to kRegSort list entries into
-//    registers, sorts them there and replays them; longer lists fall back to
-//    repeated minimum selection.
 template <bool GLOBAL_RING>
 __device__ void apply_ordered(int ce, int* head, int* tail, int ncols_local, int* st_col,
                               const int* st_slot, const float* st_w, int* st_next, float* ring,
-                              int ring_stride, int col0, int serial_max) {
+                              int ring_stride, int col0) {
   __syncthreads();
   if (ce <= kCountMax && ce <= (int)blockDim.x) {
     apply_cells<GLOBAL_RING>(ce, st_next, st_col, st_slot, st_w, ring, ring_stride, col0);
-    return;
-  }
-  if (ce > serial_max) {
-    for (int q = threadIdx.x; q < ce; q += blockDim.x) st_next[q] = atomicExch(&head[st_col[q]], q);
-    __syncthreads();
-    for (int c = threadIdx.x; c < ncols_local; c += blockDim.x) {
-      const int h = head[c];
-      if (h < 0) continue;
-      head[c] = -1;
-      int r[kRegSort];
-#pragma unroll
-      for (int i = 0; i < kRegSort; ++i) r[i] = INT_MAX;
-      int p = h;
-#pragma unroll
-      for (int i = 0; i < kRegSort; ++i) {
-        if (p >= 0) {
-          // insert p into the sorted r[0..kRegSort) (largest slot is free)
-          r[kRegSort - 1] = p;
-#pragma unroll
-          for (int k = kRegSort - 1; k > 0; --k) {
-            const int lo = min(r[k - 1], r[k]), hi = max(r[k - 1], r[k]);
-            r[k - 1] = lo;
-            r[k] = hi;
-          }
-          p = st_next[p];
-        }
-      }
-      if (p < 0) {
-#pragma unroll
-        for (int i = 0; i < kRegSort; ++i)
-          if (r[i] != INT_MAX) apply_one<GLOBAL_RING>(ring, ring_stride, col0, c, st_slot[r[i]], st_w[r[i]]);
-      } else {
-        int last = -1;
-        for (;;) {
-          int best = INT_MAX;
-          for (int x = h; x >= 0; x = st_next[x])
-            if (x > last && x < best) best = x;
-          if (best == INT_MAX) break;
-          apply_one<GLOBAL_RING>(ring, ring_stride, col0, c, st_slot[best], st_w[best]);
-          last = best;
-        }
-      }
-    }
-    __syncthreads();
     return;
   }
   {
@@ -463,52 +405,142 @@ __device__ void apply_ordered(int ce, int* head, int* tail, int ncols_local, int
   __syncthreads();
 }
 
+constexpr int kSThreads = 1024;
+enum { kSAtomic = 0, kSOrdered = 1, kSLean = 2 };  // deliveries of the tier-S kernel
+constexpr int kSRows = 4;   // fired rows of a lane: a tier-S warp takes 128 at once
+constexpr int kSAhead = 2;  // 32-event groups whose edges a tier-S warp keeps in flight
+constexpr int kSTags = 512; // bytes of a warp's own tags where every cell cannot have one
+constexpr int kSScratch = 32 * kSRows + 32 + 4;  // ints of scratch of a tier-S warp
+constexpr int kSOff = kSPtr + 1;  // ints of a staged row (odd: no bank conflicts)
+
+// Where the segment starts of the k-th staged fired row lie: lane l reads
+// rows 4 l .. 4 l + 3 of every 128, each read free of bank conflicts.
+__device__ __forceinline__ int stage_slot(int k) {
+  return (k & ~127) + (k & 3) * 32 + ((k & 127) >> 2);
+}
+
+__device__ __forceinline__ int lds_i(unsigned a) {
+  int v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float lds_f(unsigned a) { return __int_as_float(lds_i(a)); }
+__device__ __forceinline__ int lds_b(unsigned a) {
+  int v;
+  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts_i(unsigned a, int v) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sts_f(unsigned a, float v) { sts_i(a, __float_as_int(v)); }
+__device__ __forceinline__ void sts_b(unsigned a, int v) {
+  asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// Adds the events of one 32-event group whose cells (shared addresses) may
+// coincide: rank is an event's place among the group's events of its cell.
+__device__ __forceinline__ void add_ranked(bool valid, unsigned cell, float w, int rank) {
+  for (int r = 0; __any_sync(0xffffffffu, valid && rank >= r); ++r) {
+    if (valid && rank == r) sts_f(cell, __fadd_rn(lds_f(cell), w));
+    __syncwarp();
+  }
+}
+
+// Copies the segment starts of row j (and the end of its last segment) to
+// shared memory, asynchronously (the whole warp; cp.async.wait_all follows).
+__device__ __forceinline__ void stage_row(const int* __restrict__ sptr, int j, int* dst, int lane) {
+  static_assert(kSPtr == 32, "an entry per lane");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst + lane)),
+               "l"(sptr + j * kSPtr + lane)
+               : "memory");
+}
+
 // ---------------------------------------------------------------------------
-// tier S: one CTA per sample, state in shared memory
+// tier S: one CTA per sample, state in registers and shared memory
 // ---------------------------------------------------------------------------
-template <int MODE, bool EP>
-__global__ void __launch_bounds__(1024, 1) k_tier_s(FwdArgs a) {
+// Every warp owns a set of the ring's columns (kSRanges ranges of about equal
+// in-degree, hub columns spread over them) and is the only one that ever adds to their cells, so
+// the delivery of a step needs no barrier, no float atomics and no tables: the
+// warp walks the step's fired rows in ascending order, reads its own segment
+// of each row (sedges: the row stably regrouped by range; sptr: the segment
+// starts), 32 events at a time, and adds them.  Events of one 32-event group
+// that meet in a cell are added one after another in lane order; every other
+// pair of a cell's events is in program order.  That is the CPU backend's
+// (pre, edge) order: SORT, bit for bit.
+//
+// What bounds it, on a 1744-neuron net (197 k synapses, delays to 30) at 57
+// fired rows and 7000 events a step: 1.1 us of a step are three barriers and
+// the integration, 1.2 us two dependent trips to L2 (segment starts, edges),
+// and every 32 events cost about 35 cycles of the SM, two thirds of them
+// shared-memory passes over random cells (tag, ring).  8.0 us a step, 17.2 with
+// events staged 1024 at a time by a search per event and ordered through cell
+// bitmaps and a hash table; ATOMIC 4.1 us, 6.0 with the rows of a warp's list
+// fetched one after another; a 1050-neuron net with 90 short rows a step 4.3
+// us, 5.2 before.  Slower: 16 ranges and warps (too few in flight), owners that
+// add one row's segment at a time without a conflict check (130 cycles a row
+// for the chain), match.any for the conflicts (100 cycles a group), edges
+// requested 4 or 8 groups ahead in registers (they share scoreboards, so the
+// oldest waits for the newest).
+//
+// ATOMIC delivery (DEL kSAtomic) needs no order: a warp per fired row, shared
+// float atomics.  States that fill a CTA's shared memory to the brim leave no
+// room for scratch: DEL kSLean walks the segments one by one instead.
+//
+// A step: integrate (thread per neuron, the state of up to KN neurons a
+// thread in registers; KN = 0: any number, in shared memory) | fired list,
+// the fired rows' segment starts copied to shared memory with cp.async, the
+// next step's drive | deliver.
+template <int KN, bool EP, int DEL>
+__global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int scratch[40];
   __shared__ long long lscratch[40];
   __shared__ int s_q;
-  const int N = a.N, R = a.R, nc = a.ncols, noc = a.noc;
-  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = nthr >> 5;
-  const int CH = nthr;
+  constexpr int nthr = kSThreads, nwarps = nthr / 32;
+  const int N = a.N, R = a.R, nc = a.ncols, noc = a.noc, RN = R * nc;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const int nch = KN ? KN : (N + nthr - 1) / nthr;  // neurons of a thread
   float* ring = reinterpret_cast<float*>(smem_raw);
-  float* v = ring + (size_t)R * nc;
-  int* refr = reinterpret_cast<int*>(v + N);
-  float* ext = reinterpret_cast<float*>(refr + N);
-  int* fired = reinterpret_cast<int*>(ext + N);
-  int* counts = fired + N;
-  int* pref = counts + noc;
-  // the column-list apply's arrays (SORT without the cell table); the lean
-  // table layout of the e-prop kernel keeps only the staged weights of them
-  // (the forward keeps the fixed layout, measured faster)
-  const bool lists = MODE == MODE_SORT && !(EP && a.s_lean);
-  int* head = pref + (N + 1);
-  int* tail = head + (lists ? nc : 0);
-  int* st_col = tail + (lists ? nc : 0);
-  int* st_slot = st_col + (lists ? CH : 0);
-  float* st_w = reinterpret_cast<float*>(st_slot + (lists ? CH : 0));
-  int* st_next = reinterpret_cast<int*>(st_w + CH);
-  // e-prop: pre-synaptic trace per neuron, surrogate psi per ring column
-  float* tr = MODE == MODE_SORT ? reinterpret_cast<float*>(st_next + (lists ? CH : 0))
-                                : reinterpret_cast<float*>(counts + noc);
-  float* psi = tr + N;
-  // SORT with a.s_table: the per-cell table for whole chunks (kSTable keys,
-  // kSTable list heads, CH links)
-  int* ctab = reinterpret_cast<int*>(EP ? psi + nc : tr);
-  // s_table 2: bitmaps of the ring's cells after the table's links, two
-  // pairs (seen, more than once) used by alternate chunks
-  const int nbw = (int)(((size_t)R * nc + 31) / 32);
-  unsigned* cbits = reinterpret_cast<unsigned*>(ctab + 2 * kSTable + CH);
-  if (MODE == MODE_SORT && a.s_table) {
-    for (int i = tid; i < 2 * kSTable; i += nthr) ctab[i] = 0;  // ordered by the loop's first barrier
-    if (a.s_table == 2)
-      for (int i = tid; i < 4 * nbw; i += nthr) cbits[i] = 0u;
+  float* ext = ring + RN;
+  int* counts = reinterpret_cast<int*>(ext + N);
+  int* wcnt = counts + noc;  // [nch][nwarps] fired neurons of each 32
+  float* sv = reinterpret_cast<float*>(wcnt + nch * nwarps);  // KN == 0 only
+  int* srefr = reinterpret_cast<int*>(sv + (KN ? 0 : N));
+  float* tr = reinterpret_cast<float*>(srefr + (KN ? 0 : N));  // inline eligibility only
+  const bool inl = EP && a.elig;
+  float* psi = tr + (inl ? N : 0);
+  int* off = reinterpret_cast<int*>(psi + (inl ? nc : 0));  // [s_cap][kSOff] staged rows
+  // per warp: segment offsets and segment marks
+  int* scr0 = off + (DEL != kSOrdered ? 0 : a.s_cap * kSOff);
+  int* scr = scr0 + (DEL != kSOrdered ? 0 : warp * kSScratch);
+  unsigned* mark = reinterpret_cast<unsigned*>(scr + 32 * kSRows);
+  unsigned short* fired = reinterpret_cast<unsigned short*>(scr0 + (DEL != kSOrdered ? 0 : nwarps * kSScratch));
+  // a byte per cell, or kSTags per warp
+  unsigned char* tag = reinterpret_cast<unsigned char*>(fired + N) + (a.s_tmask == kSTags - 1 ? warp * kSTags : 0);
+  const int tmask = a.s_tmask;
+  const LifP lif = a.lif;
+  const float thr = lif.thr;
+  // the delivery's arrays as shared addresses
+  const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring);
+  const unsigned off_w = (unsigned)__cvta_generic_to_shared(off + lane * kSOff + warp);
+  const unsigned scr_s = (unsigned)__cvta_generic_to_shared(scr);
+  const unsigned mark_s = (unsigned)__cvta_generic_to_shared(mark);
+  const unsigned tag_s = (unsigned)__cvta_generic_to_shared(tag);
+  const unsigned upto = below | (1u << lane);
+  const uint2* __restrict__ sed = a.sedges;
+
+  float vr[KN ? KN : 1];
+  int rf[KN ? KN : 1], colr[KN ? KN : 1];
+  unsigned outm = 0;  // bit c: the neuron is an output with a channel
+#pragma unroll
+  for (int c = 0; c < nch; ++c) {
+    const int j = c * nthr + tid;
+    if (KN) colr[KN ? c : 0] = j < N ? a.col_of[j] : -1;
+    if (j < N && a.out_ch[j] >= 0) outm |= 1u << c;
   }
+  const unsigned rom = a.ro_on ? outm : 0u;  // bit c: a leaky readout unit
 
   for (;;) {
     if (tid == 0) s_q = (int)atomicAdd(&a.ctl[1], 1u);
@@ -517,101 +549,143 @@ __global__ void __launch_bounds__(1024, 1) k_tier_s(FwdArgs a) {
     if (q >= a.B) break;
     const int b = a.order[q];
     const int T = a.steps[b];
-    for (int i = tid; i < R * nc; i += nthr) ring[i] = 0.f;
+    for (int i = tid; i < RN; i += nthr) ring[i] = 0.f;
     for (int i = tid; i < N; i += nthr) {
-      v[i] = 0.f;
-      refr[i] = 0;
       ext[i] = 0.f;
-      if (EP) tr[i] = 0.f;
+      if (!KN) {
+        sv[i] = 0.f;
+        srefr[i] = 0;
+      }
+      if (inl) tr[i] = 0.f;
+    }
+    if (KN) {
+#pragma unroll
+      for (int c = 0; c < KN; ++c) {
+        vr[c] = 0.f;
+        rf[c] = 0;
+      }
     }
     for (int i = tid; i < noc; i += nthr) counts[i] = 0;
-    if (lists)
-      for (int i = tid; i < nc; i += nthr) {
-        head[i] = -1;
-        tail[i] = -1;
-      }
     __syncthreads();
     const int* sp = a.sched_ptr + a.sptr_off[b];
-    uint32_t* rast = a.raster ? a.raster + a.raster_off[b] : nullptr;
-    long long my_spikes = 0, my_events = 0;
-    int s0 = 0;
-    __shared__ int s_bc[2][32];  // ballot_compact_1 buffers, alternated
-    int bcp = 0;
-    // the drive of step t: thread i holds entry i of the step's schedule in
-    // registers, loaded a step ahead (entries beyond blockDim.x are read in
-    // the step itself); a step's entries name distinct neurons
-    int pf_lo = T > 0 ? sp[0] : 0, pf_hi = T > 0 ? sp[1] : 0, pf_nid = -1;
+    uint32_t* rast = a.raster ? a.raster + a.raster_off[b] + warp : nullptr;
+    float* psi_t = EP && a.psi_hist ? a.psi_hist + (size_t)b * a.psi_T * nc : nullptr;
+    long long n_spikes = 0, n_events = 0;  // of the sample / of this warp's columns
+    int s0n = 0;                           // first cell of the current slot
+    // the drive: a step's entries name distinct neurons; thread i holds entry
+    // i of the next step's in registers, loaded a step ahead from a range
+    // whose end was itself loaded a step earlier (entries beyond blockDim.x
+    // are read when they are stored)
+    int p_lo = 0, p_hi = 0, p_nx = 0, pf_nid = -1;
     float pf_ext = 0.f;
-    if (pf_lo + tid < pf_hi) {
-      pf_nid = a.sched_nid[pf_lo + tid];
-      pf_ext = a.sched_ext[pf_lo + tid];
+    auto fetch_drive = [&]() {
+      pf_nid = -1;
+      if (p_lo + tid < p_hi) {
+        pf_nid = a.sched_nid[p_lo + tid];
+        pf_ext = a.sched_ext[p_lo + tid];
+      }
+    };
+    auto store_drive = [&]() {
+      if (pf_nid >= 0) ext[pf_nid] = pf_ext;
+      for (int k = p_lo + nthr + tid; k < p_hi; k += nthr) ext[a.sched_nid[k]] = a.sched_ext[k];
+    };
+    if (T > 0) {
+      p_lo = sp[0];
+      p_hi = sp[1];
+      fetch_drive();
+      store_drive();
+      p_lo = p_hi;
+      p_hi = sp[min(2, T)];
+      fetch_drive();  // step 1
+      p_nx = sp[min(3, T)];
+      __syncthreads();
     }
     for (int t = 0; t < T; ++t) {
-      float* slot = ring + (size_t)s0 * nc;
-      if (pf_nid >= 0) ext[pf_nid] = pf_ext;
-      for (int k = pf_lo + nthr + tid; k < pf_hi; k += nthr) ext[a.sched_nid[k]] = a.sched_ext[k];
-      __syncthreads();
-      pf_nid = -1;
-      if (t + 1 < T) {
-        pf_lo = sp[t + 1];
-        pf_hi = sp[t + 2];
-        if (pf_lo + tid < pf_hi) {
-          pf_nid = a.sched_nid[pf_lo + tid];
-          pf_ext = a.sched_ext[pf_lo + tid];
-        }
-      }
-      // integrate / fire, ascending fired list via ballot compaction
-      int nf = 0;
-      for (int base = 0; base < N; base += nthr) {
-        const int j = base + tid;
-        int f = 0;
+      unsigned fm = 0;  // bit c: this thread's neuron of chunk c fired
+#pragma unroll
+      for (int c = 0; c < nch; ++c) {
+        const int j = c * nthr + tid;
+        bool f = false;
         if (j < N) {
-          float vv = v[j];
-          int rr = refr[j];
+          float vv = KN ? vr[KN ? c : 0] : sv[j];
+          int rr = KN ? rf[KN ? c : 0] : srefr[j];
+          const int col = KN ? colr[KN ? c : 0] : a.col_of[j];
           const float e = ext[j];
           ext[j] = 0.f;
-          const int c = a.col_of[j];
           float rin = 0.f;
-          if (c >= 0) {
-            rin = slot[c];
-            slot[c] = 0.f;
+          if (col >= 0) {
+            rin = ring[s0n + col];
+            ring[s0n + col] = 0.f;
           }
-          float vpre;
-          const int oc = a.out_ch[j];
-          f = a.ro_on && oc >= 0 ? readout_step(a.ro_decay, vv, e, rin, &vpre)
-                                 : lif_step(a.lif, vv, rr, e, rin, &vpre);
-          v[j] = vv;
-          refr[j] = rr;
+          // lif_step / readout_step without branches
+          const bool ro = (rom >> c) & 1u, idle = !ro && rr > 0;
+          const float nv = lif_integrate(vv, ro ? a.ro_decay : lif.decay, e, rin);
+          f = !ro && !idle && nv >= thr;
+          const float vf = lif.reset_mode ? __fsub_rn(nv, thr) : lif.reset;
+          vv = idle ? lif.reset : f ? vf : nv;
+          rr = idle ? rr - 1 : f ? lif.refractory : rr;
+          if (KN) {
+            vr[KN ? c : 0] = vv;
+            rf[KN ? c : 0] = rr;
+          } else {
+            sv[j] = vv;
+            srefr[j] = rr;
+          }
           if (EP) {
             // cuda_trainer.cu:93-95: triangular surrogate and pre trace
-            const float thr = a.lif.thr;
-            const float dd = __fdiv_rn(fabsf(__fsub_rn(vpre, thr)), thr > 0.f ? thr : 1.f);
-            if (c >= 0) {
+            if (col >= 0) {
+              float dd = fabsf(__fsub_rn(idle ? lif.reset : nv, thr));
+              if (thr > 0.f && thr != 1.f) dd = __fdiv_rn(dd, thr);  // x / 1 = x
               const float ps = dd < 1.f ? __fmul_rn(a.gamma, __fsub_rn(1.f, dd)) : 0.f;
-              psi[c] = ps;
-              if (a.psi_hist) a.psi_hist[((size_t)b * a.psi_T + t) * nc + c] = ps;
+              if (inl) psi[col] = ps;
+              if (psi_t) psi_t[col] = ps;
             }
-            tr[j] = __fadd_rn(__fmul_rn(a.trace_decay, tr[j]),
-                              __fmul_rn(__fsub_rn(1.f, a.trace_decay), f ? 1.f : 0.f));
+            if (inl)
+              tr[j] = __fadd_rn(__fmul_rn(a.trace_decay, tr[j]),
+                                __fmul_rn(__fsub_rn(1.f, a.trace_decay), f ? 1.f : 0.f));
             if (f && a.fires) atomicAdd(&a.fires[j], 1ull);
           }
           if (f) {
-            ++my_spikes;
-            my_events += a.row_ptr[j + 1] - a.row_ptr[j];
-            if (oc >= 0) atomicAdd(&counts[oc], 1);
+            fm |= 1u << c;
+            if ((outm >> c) & 1u) atomicAdd(&counts[a.out_ch[j]], 1);
           }
         }
-        int tot;
-        unsigned m;
-        const int pos = ballot_compact_1(f, s_bc[bcp], &tot, &m);
-        bcp ^= 1;
-        if (rast && lane == 0 && base + warp * 32 < N)
-          rast[(size_t)t * a.W + ((base + warp * 32) >> 5)] = m;
-        if (f) fired[nf + pos] = j;
-        nf += tot;
+        const unsigned m = __ballot_sync(0xffffffffu, f);
+        if (lane == 0) {
+          wcnt[c * nwarps + warp] = __popc(m);
+          if (rast && c * nthr + warp * 32 < N) rast[c * nwarps] = m;
+        }
       }
+      if (rast) rast += a.W;
+      if (EP && psi_t) psi_t += nc;
       __syncthreads();
-      if (EP && a.elig) {
+      // ascending fired list; the segment starts of the first s_cap fired rows
+      int nf = 0;
+#pragma unroll
+      for (int c = 0; c < nch; ++c) {
+        // (fired of the chunk's earlier warps, fired of the chunk) in one sum
+        const int n = lane < nwarps ? wcnt[c * nwarps + lane] : 0;
+        const unsigned both =
+            __reduce_add_sync(0xffffffffu, (unsigned)((lane < warp ? n : 0) | (n << 16)));
+        int rk = nf + (int)(both & 0xffffu);
+        nf += (int)(both >> 16);
+        const bool f = (fm >> c) & 1u;
+        unsigned m = __ballot_sync(0xffffffffu, f);
+        if (!m) continue;
+        if (f) fired[rk + __popc(m & below)] = (unsigned short)(c * nthr + tid);
+        if (DEL == kSOrdered)
+          for (; m && rk < a.s_cap; m &= m - 1u, ++rk)
+            stage_row(a.sptr, c * nthr + warp * 32 + __ffs(m) - 1, off + stage_slot(rk) * kSOff, lane);
+      }
+      n_spikes += nf;
+      store_drive();
+      p_lo = p_hi;
+      p_hi = p_nx;
+      fetch_drive();
+      p_nx = sp[min(t + 4, T)];
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      if (inl) {
         // cuda_trainer.cu:105-112: E[b,s] += psi[post] * tr[pre]; rows whose
         // trace is exactly zero add +0 and are skipped (trainer.cpp:243-244)
         float* Eb = a.elig + (size_t)b * a.S;
@@ -625,165 +699,192 @@ __global__ void __launch_bounds__(1024, 1) k_tier_s(FwdArgs a) {
           }
         }
       }
-      if (MODE != MODE_SORT) {
-        // warp per fired row; two edges per lane per 128-bit load
+      const unsigned s0b = ring_s + 4u * s0n, end_s = ring_s + 4u * RN;
+      auto cell_at = [&](unsigned x) {  // shared address of the cell of an edge
+        const unsigned c = s0b + x;
+        return c >= end_s ? c - 4u * RN : c;
+      };
+      if (DEL == kSAtomic) {
+        // a warp per fired row; two edges per lane per 128-bit load, the
+        // loads of up to 256 edges before the first add
         for (int k = warp; k < nf; k += nwarps) {
           const int j = fired[k];
           const int rs = a.row_ptr[j], re = a.row_ptr[j + 1];
-          for (int e = (rs & ~1) + 2 * lane; e < re; e += 64) {
-            const uint4 pr = *reinterpret_cast<const uint4*>(a.edges + e);
-            if (e >= rs) {
-              const uint2 ed = make_uint2(pr.x, pr.y);
-              atomicAdd(&ring[(size_t)ring_slot(s0, edge_delay(ed), R) * nc + edge_col(ed)], edge_w(ed));
+          n_events += re - rs;
+          for (int e0 = rs & ~1; e0 < re; e0 += 256) {
+            uint4 pr[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int e = e0 + 64 * u + 2 * lane;
+              pr[u] = e < re ? *reinterpret_cast<const uint4*>(a.edges + e) : make_uint4(0u, 0u, 0u, 0u);
             }
-            if (e + 1 < re) {
-              const uint2 ed = make_uint2(pr.z, pr.w);
-              atomicAdd(&ring[(size_t)ring_slot(s0, edge_delay(ed), R) * nc + edge_col(ed)], edge_w(ed));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int e = e0 + 64 * u + 2 * lane;
+              const uint2 x = make_uint2(pr[u].x, pr[u].y), y = make_uint2(pr[u].z, pr[u].w);
+              auto cell = [&](uint2 ed) {
+                const int c = s0n + edge_delay(ed) * nc + edge_col(ed);
+                return ring + (c >= RN ? c - RN : c);
+              };
+              if (e >= rs && e < re) atomicAdd(cell(x), edge_w(x));
+              if (e + 1 < re) atomicAdd(cell(y), edge_w(y));
             }
           }
         }
-      } else {
-        int base = 0;
-        for (int k0 = 0; k0 < nf; k0 += nthr) {
-          const int k = k0 + tid;
-          int len = 0;
-          if (k < nf) {
-            const int rs = a.row_ptr[fired[k]];
-            len = a.row_ptr[fired[k] + 1] - rs;
-            fired[k] = rs;  // row start from here on (the list is not used again this step)
-          }
-          int tot;
-          const int ex = block_exclusive_scan(len, scratch, &tot);
-          if (k < nf) pref[k] = base + ex;
-          base += tot;
-        }
-        __syncthreads();
-        const int E = base;
-        if (a.s_table) {
-          // per-cell apply of whole chunks (CH = blockDim.x: thread q stages
-          // event q of the chunk and enters it in its cell's list; staging
-          // order is the (pre, edge) order)
-          // the table is all zero between chunks: every cell's owner clears
-          // its entry once it has applied the cell (nobody else reads it)
-          // thread q's edge of the next chunk is requested before this
-          // chunk's cells are applied, so the load overlaps the apply
-          const int q = tid;
-          auto edge_of = [&](int e) {
-            const int k = upper_index(pref, nf, e);
-            return a.edges[fired[k] + (e - pref[k])];
-          };
-          uint2 ed_next = q < E ? edge_of(q) : make_uint2(0u, 0u);
-          if (a.s_table == 2) {
-            // Only cells hit more than once in a chunk need the table: every
-            // event marks its cell in the chunk's bitmap pair (a second mark
-            // sets the "more than once" bit); after one barrier a cell hit
-            // once takes its event directly and the others go through the
-            // table, applied after a second barrier.  Each event clears its
-            // cell's seen word once it has read it (the events of shared cells
-            // also their "more" word); the pairs alternate, so a
-            // chunk's marks never meet the previous chunk's clears.  (A
-            // shared-memory atomic add for the single events and bulk clears
-            // of the idle pair both measured slower.)
-            int pair = 0;
-            for (int e0 = 0; e0 < E; e0 += CH, pair ^= 1) {
-              const int ce = min(CH, E - e0);
-              const uint2 ed = ed_next;
-              unsigned* seen = cbits + (size_t)pair * 2 * nbw;
-              unsigned* more = seen + nbw;
-              int c = 0, sl = 0, bw = 0;
-              unsigned bm = 0, h = 0;
-              float w = 0.f;
-              if (q < ce) {
-                sl = ring_slot(s0, edge_delay(ed), R);
-                c = edge_col(ed);
-                w = edge_w(ed);
-                const int bit = sl * nc + c;
-                bw = bit >> 5;
-                bm = 1u << (bit & 31);
-                if (atomicOr(&seen[bw], bm) & bm) atomicOr(&more[bw], bm);
+      } else if (DEL == kSLean) {
+        // lane l: this warp's segment of fired row k0 + l, one after another
+        if (warp < kSRanges)
+          for (int k0 = 0; k0 < nf; k0 += 32) {
+            int st = 0, ln = 0;
+            if (k0 + lane < nf) {
+              const int* op = a.sptr + fired[k0 + lane] * kSPtr + warp;
+              st = op[0];
+              ln = op[1] - st;
+            }
+            for (unsigned ne = __ballot_sync(0xffffffffu, ln > 0); ne; ne &= ne - 1u) {
+              const int l = __ffs(ne) - 1;
+              const int s = __shfl_sync(0xffffffffu, st, l), n = __shfl_sync(0xffffffffu, ln, l);
+              n_events += n;
+              for (int e0 = 0; e0 < n; e0 += 32) {
+                const bool valid = e0 + lane < n;
+                const uint2 ed = valid ? a.sedges[s + e0 + lane] : make_uint2(0u, 0u);
+                const unsigned cell = cell_at(ed.x);
+                const unsigned peers = __match_any_sync(0xffffffffu, valid ? (int)cell : -1 - lane);
+                add_ranked(valid, cell, __uint_as_float(ed.y), __popc(peers & below));
               }
-              // the next chunk's edge: its row search overlaps the marks and
-              // the barrier, its load the apply
-              if (e0 + CH + q < E) ed_next = edge_of(e0 + CH + q);
-              __syncthreads();
-              bool first = false, shared_cell = false;
-              if (q < ce) {
-                shared_cell = (more[bw] & bm) != 0u;
-                if (!shared_cell) {
-                  apply_one<false>(ring, nc, 0, c, sl, w);
-                } else {
-                  st_w[q] = w;
-                  h = cell_insert<kSTable>(ctab, ctab + 2 * kSTable, q, c, sl, &first);
+            }
+          }
+      } else {
+        for (int r0 = 0;;) {
+          const int nb = min(a.s_cap, nf - r0);
+          for (int k0 = 0; k0 < nb && warp < kSRanges; k0 += 32 * kSRows) {
+            // lane l: this warp's segments of kSRows consecutive fired rows
+            int st[kSRows], ln[kSRows], sum = 0, sg = 0;
+#pragma unroll
+            for (int i = 0; i < kSRows; ++i) {
+              st[i] = ln[i] = 0;
+              if (k0 + lane * kSRows + i < nb) {
+                const unsigned op = off_w + 4u * ((k0 + i * 32) * kSOff);
+                st[i] = lds_i(op);
+                ln[i] = lds_i(op + 4u) - st[i];
+              }
+              sum += ln[i];
+              sg += __popc(__ballot_sync(0xffffffffu, ln[i] > 0) & below);  // earlier lanes' segments
+            }
+            const int total = __reduce_add_sync(0xffffffffu, sum);
+            n_events += total;
+            int pos = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const int y = __shfl_up_sync(0xffffffffu, pos, o);
+              if (lane >= o) pos += y;
+            }
+            pos -= sum;    // events of earlier lanes
+            unsigned segs = scr_s - 4u;  // last segment begun before the group
+            for (int w0 = 0; w0 < total; w0 += 1024) {
+              // bit q - w0 of the marks: a segment begins at event q; event q
+              // of a segment is edge st - (its first event) + q
+              __syncwarp();
+              sts_i(mark_s + 4u * lane, 0);
+              __syncwarp();
+              int p = pos - w0;
+              unsigned g = scr_s + 4u * sg;
+#pragma unroll
+              for (int i = 0; i < kSRows; ++i) {
+                if (ln[i] > 0) {
+                  sts_i(g, st[i] - (p + w0));
+                  g += 4u;
+                  if ((unsigned)p < 1024u) atomicOr(&mark[p >> 5], 1u << (p & 31));
+                }
+                p += ln[i];
+              }
+              __syncwarp();
+              const int end = min(total, w0 + 1024);
+              int ql = w0 + lane;  // this lane's event of the group loaded next
+              unsigned mk = mark_s;
+              // edges are requested kSAhead groups before they are applied
+              uint2 ed[kSAhead];
+              auto load = [&](uint2& x) {
+                const unsigned M = (unsigned)lds_i(mk);  // (the group behind the last reads a spare word)
+                mk += 4u;
+                if (ql < end) x = sed[lds_i(segs + 4u * __popc(M & upto)) + ql];
+                segs += 4u * __popc(M);
+                ql += 32;
+              };
+#pragma unroll
+              for (int u = 0; u < kSAhead; ++u)
+                if (w0 + 32 * u < end) load(ed[u]);
+              for (int q0 = w0; q0 < end; q0 += 32 * kSAhead) {
+#pragma unroll
+                for (int u = 0; u < kSAhead; ++u) {
+                  const int qu = q0 + 32 * u;
+                  if (qu >= end) break;
+                  const bool valid = qu + lane < end;
+                  const unsigned cell = cell_at(ed[u].x);
+                  const float w = __uint_as_float(ed[u].y);
+                  if (qu + 32 * kSAhead < end) load(ed[u]);
+                  // Every event marks its cell's tag; whoever finds another's
+                  // mark there shares its cell with an event of this group.
+                  const unsigned tg = tag_s + (((cell - ring_s) >> 2) & tmask);
+                  if (valid) sts_b(tg, lane);
+                  __syncwarp();
+                  int mk = valid ? lds_b(tg) : lane;
+                  if (!__any_sync(0xffffffffu, mk != lane)) {
+                    if (valid) sts_f(cell, __fadd_rn(lds_f(cell), w));
+                    __syncwarp();
+                    continue;
+                  }
+                  // Those of one tag one after another, the earliest first: an
+                  // event that finds a later one's mark marks again (the
+                  // lowest lane's mark is the one that stays, so this hardly
+                  // ever repeats), whoever finds its own mark adds.
+                  bool pend = valid;
+                  for (;;) {
+                    while (__any_sync(0xffffffffu, pend && mk > lane)) {
+                      __syncwarp();
+                      if (pend && mk > lane) sts_b(tg, lane);
+                      __syncwarp();
+                      if (pend) mk = lds_b(tg);
+                    }
+                    if (pend && mk == lane) {
+                      sts_f(cell, __fadd_rn(lds_f(cell), w));
+                      pend = false;
+                    }
+                    __syncwarp();
+                    if (!__any_sync(0xffffffffu, pend)) break;
+                    if (pend) sts_b(tg, lane);
+                    __syncwarp();
+                    if (pend) mk = lds_b(tg);
+                  }
                 }
               }
-              __syncthreads();
-              if (q < ce) {
-                seen[bw] = 0u;
-                if (shared_cell) more[bw] = 0u;  // other words of `more` stayed zero
-              }
-              if (first) {
-                cell_apply<false, false, kSTable>(ctab, ctab + 2 * kSTable, nullptr, st_w, h, q, c, sl, ring,
-                                                  nc, 0);
-                ctab[h] = 0;
-                ctab[kSTable + h] = 0;
-              }
             }
-            // the step's closing barrier orders the last chunk's apply
-          } else
-          for (int e0 = 0; e0 < E; e0 += CH) {
-            const int ce = min(CH, E - e0);
-            const uint2 ed = ed_next;
-            int c = 0, sl = 0;
-            unsigned h = 0;
-            bool first = false;
-            if (q < ce) {
-              sl = ring_slot(s0, edge_delay(ed), R);
-              c = edge_col(ed);
-              st_w[q] = edge_w(ed);
-              h = cell_insert<kSTable>(ctab, ctab + 2 * kSTable, q, c, sl, &first);
-            }
-            __syncthreads();
-            if (e0 + CH + q < E) ed_next = edge_of(e0 + CH + q);
-            if (first) {
-              cell_apply<false, false, kSTable>(ctab, ctab + 2 * kSTable, nullptr, st_w, h, q, c, sl, ring,
-                                                nc, 0);
-              ctab[h] = 0;
-              ctab[kSTable + h] = 0;
-            }
-            __syncthreads();
           }
-        } else
-        for (int e0 = 0; e0 < E; e0 += CH) {
-          const int ce = min(CH, E - e0);
-          for (int qq = tid; qq < ce; qq += nthr) {
-            const int e = e0 + qq;
-            const int k = upper_index(pref, nf, e);
-            const uint2 ed = a.edges[fired[k] + (e - pref[k])];
-            st_slot[qq] = ring_slot(s0, edge_delay(ed), R);
-            st_w[qq] = edge_w(ed);
-            st_col[qq] = edge_col(ed);
-          }
-          if (ce <= kCountMax)  // apply_cells' table (st_next has CH = 1024 entries)
-            for (int i = tid; i < 2 * kCellTable; i += nthr) st_next[i] = 0;
+          r0 += a.s_cap;
+          if (r0 >= nf) break;
+          // more fired rows than s_cap: the next ones' segment starts
           __syncthreads();
-          apply_ordered<false>(ce, head, tail, nc, st_col, st_slot, st_w, st_next, ring, nc, 0,
-                               kCountMax);
+          for (int k = warp; k < min(a.s_cap, nf - r0); k += nwarps)
+            stage_row(a.sptr, fired[r0 + k], off + stage_slot(k) * kSOff, lane);
+          asm volatile("cp.async.wait_all;" ::: "memory");
           __syncthreads();
         }
       }
       __syncthreads();
-      s0 = (s0 + 1 == R) ? 0 : s0 + 1;
+      s0n = s0n + nc == RN ? 0 : s0n + nc;
     }
     for (int i = tid; i < noc; i += nthr) a.counts[(size_t)b * noc + i] = counts[i];
-    if (a.vfinal)
-      for (int i = tid; i < N; i += nthr) a.vfinal[(size_t)b * N + i] = v[i];
-    if (a.ro_on)
-      for (int i = tid; i < N; i += nthr)
-        if (a.ro_rank[i] >= 0) a.ro_v[(size_t)b * a.n_ro + a.ro_rank[i]] = v[i];
-    const long long ts = block_sum_ll(my_spikes, lscratch);
-    const long long te = block_sum_ll(my_events, lscratch);
+#pragma unroll
+    for (int c = 0; c < nch; ++c) {
+      const int j = c * nthr + tid;
+      if (j >= N) break;
+      const float vv = KN ? vr[KN ? c : 0] : sv[j];
+      if (a.vfinal) a.vfinal[(size_t)b * N + j] = vv;
+      if (a.ro_on && a.ro_rank[j] >= 0) a.ro_v[(size_t)b * a.n_ro + a.ro_rank[j]] = vv;
+    }
+    const long long te = block_sum_ll(lane == 0 ? n_events : 0, lscratch);
     if (tid == 0) {
-      a.spikes[b] = (unsigned long long)ts;
+      a.spikes[b] = (unsigned long long)n_spikes;
       a.events[b] = (unsigned long long)te;
     }
     __syncthreads();
@@ -1107,7 +1208,7 @@ __device__ void phase_b_scan(const FwdArgs& a, const GSmem& sm, int* scratch, in
       if (ce <= kCountMax)  // apply_cells' table
         for (int i = tid; i < 2 * kCellTable; i += nthr) sm.st_next[i] = 0;
       apply_ordered<!RSM>(ce, sm.head, sm.tail, cb1 - cb0, sm.st_col, sm.st_slot, sm.st_w,
-                          sm.st_next, rb, stride, col0, kGChunk);
+                          sm.st_next, rb, stride, col0);
     }
   }
 }
@@ -1313,7 +1414,7 @@ __device__ void phase_b(const FwdArgs& a, const GSmem& sm, int* scratch, int k, 
         if (ce <= kCountMax)  // apply_cells' table
           for (int i = tid; i < 2 * kCellTable; i += nthr) sm.st_next[i] = 0;
         apply_ordered<!RSM>(ce, sm.head, sm.tail, cb1 - cb0, sm.st_col, sm.st_slot, sm.st_w,
-                            sm.st_next, rb, stride, col0, kGChunk);
+                            sm.st_next, rb, stride, col0);
       } else {
         __syncthreads();
       }
@@ -1477,7 +1578,7 @@ static FwdArgs make_args(Run* r, const snc_lif* lif) {
   a.P = g->P; a.BS = g->BS; a.G = g->G;
   a.row_ptr = g->row_ptr; a.edges = g->edges; a.gedges = g->gedges; a.gptr = g->gptr;
   a.groups = g->groups; a.col_of = g->col_of; a.out_ch = g->out_ch; a.colbase = g->colbase;
-  a.ibase = g->ibase;
+  a.ibase = g->ibase; a.sedges = g->sedges; a.sptr = g->sptr;
   a.B = in->B; a.order = in->order; a.steps = in->steps; a.sptr_off = in->sptr_off;
   a.stepbase = in->stepbase;
   a.sched_ptr = in->sched_ptr; a.sched_nid = in->sched_nid; a.sched_ext = in->sched_ext;
@@ -1538,55 +1639,74 @@ static int optin_smem() {
   return optin;
 }
 
-template <int MODE, bool EP>
-static int launch_tier_s_kernel(const Graph* g, int B, const FwdArgs& a_in, cudaStream_t st) {
-  const int nthr = 1024;
-  FwdArgs a = a_in;
-  size_t smem = tier_s_bytes(g->N, g->ncols, g->R, a.noc, MODE, EP, nthr);
-  SNCB_CUDA(cudaFuncSetAttribute(k_tier_s<MODE, EP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  SNCB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tier_s<MODE, EP>, nthr, smem));
-  a.s_table = 0;
-  a.s_lean = 0;
-  if (MODE == MODE_SORT) {
-    // the per-cell table (and the cell bitmaps with it) when it fits without
-    // costing a CTA per SM; the richest layout that fits, the full one before
-    // the lean one (e-prop only)
-    for (int v = 0; v < 4 && !a.s_table; ++v) {
-      const int tab = 2 - v / 2;
-      const bool lean = (v & 1) != 0;
-      if (lean && !EP) continue;
-      const size_t smem_t = tier_s_bytes(g->N, g->ncols, g->R, a.noc, MODE, EP, nthr, tab, lean);
-      int per_sm_t = 0;
-      if ((int)smem_t <= optin_smem() &&
-          cudaFuncSetAttribute(k_tier_s<MODE, EP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t) ==
-              cudaSuccess &&
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_t, k_tier_s<MODE, EP>, nthr, smem_t) ==
-              cudaSuccess &&
-          per_sm_t >= per_sm && per_sm_t >= 1) {
-        smem = smem_t;
-        a.s_table = tab;
-        a.s_lean = lean ? 1 : 0;
-      } else {
-        cudaGetLastError();
+// Launch shape of the tier-S kernel: neurons of a thread held in registers
+// (1, 2 or 4; 0: state in shared memory), the delivery, fired rows staged at
+// once, mask of the conflict tags, bytes of dynamic shared memory.
+struct SPlan {
+  int kn, del, cap, tmask;
+  size_t smem;
+};
+
+static SPlan tier_s_layout(const Graph* g, int noc, bool inl, int mode, size_t budget) {
+  const int nch = std::max(1, (g->N + kSThreads - 1) / kSThreads);
+  const size_t cells = (size_t)g->R * g->ncols, nw = kSThreads / 32;
+  SPlan p{nch <= 1 ? 1 : nch <= 2 ? 2 : nch <= 4 ? 4 : 0, kSAtomic, 0, 0, 0};
+  auto base = [&](int kn) {
+    return (cells + g->N + noc + (size_t)(kn ? kn : nch) * nw + (kn ? 0 : 2 * (size_t)g->N) +
+            (inl ? (size_t)g->N + g->ncols : 0)) * 4 + (size_t)g->N * 2 + 16;
+  };
+  p.smem = base(p.kn);
+  if (mode != MODE_SORT) return p;
+  p.del = kSOrdered;
+  const size_t b0 = p.smem + nw * kSScratch * 4;
+  // a tag per cell before tags per warp (their false conflicts cost more than
+  // a second round of staging), then the larger stage
+  for (const bool exact : {true, false})
+    for (const int cap : {256, 128}) {
+      const size_t need = b0 + (size_t)cap * kSOff * 4 + (exact ? cells : nw * kSTags);
+      if (need <= budget) {
+        p.cap = cap;
+        p.tmask = exact ? INT_MAX : kSTags - 1;
+        p.smem = need;
+        return p;
       }
     }
-    if (!a.s_table)
-      SNCB_CUDA(cudaFuncSetAttribute(k_tier_s<MODE, EP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  }
+  p.kn = 0;
+  p.del = kSLean;
+  p.smem = base(0);
+  return p;
+}
+
+template <bool EP>
+static int launch_tier_s(const Graph* g, int B, int mode, const FwdArgs& a_in, cudaStream_t st) {
+  FwdArgs a = a_in;
+  using Kern = void (*)(FwdArgs);
+  auto pick = [](int kn, int del) -> Kern {
+    if (del == kSLean) return k_tier_s<0, EP, kSLean>;
+    if (del == kSAtomic)
+      return kn == 1 ? k_tier_s<1, EP, kSAtomic> : kn == 2 ? k_tier_s<2, EP, kSAtomic>
+             : kn == 4 ? k_tier_s<4, EP, kSAtomic> : k_tier_s<0, EP, kSAtomic>;
+    return kn == 1 ? k_tier_s<1, EP, kSOrdered> : kn == 2 ? k_tier_s<2, EP, kSOrdered>
+           : kn == 4 ? k_tier_s<4, EP, kSOrdered> : k_tier_s<0, EP, kSOrdered>;
+  };
+  cudaFuncAttributes fa{};
+  SNCB_CUDA(cudaFuncGetAttributes(&fa, pick(2, kSOrdered)));
+  const size_t budget = (size_t)optin_smem() - fa.sharedSizeBytes;
+  const SPlan p = tier_s_layout(g, a.noc, EP && a.elig, mode, budget);
+  a.s_cap = p.cap;
+  a.s_tmask = p.tmask;
+  const Kern kern = pick(p.kn, p.del);
+  SNCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+  int per_sm = 0;
+  SNCB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSThreads, p.smem));
   if (per_sm < 1) {
     set_error("tier S does not fit on an SM");
     return SNC_B200_EUNSUPPORTED;
   }
   const int grid = std::max(1, std::min(B, per_sm * g->sm_count));
-  k_tier_s<MODE, EP><<<grid, nthr, smem, st>>>(a);
+  kern<<<grid, kSThreads, p.smem, st>>>(a);
   SNCB_CUDA(cudaGetLastError());
   return SNC_B200_OK;
-}
-
-template <int MODE>
-static int launch_tier_s(Run* r, const FwdArgs& a, cudaStream_t st) {
-  return launch_tier_s_kernel<MODE, false>(r->g, r->in->B, a, st);
 }
 
 // e-prop forward of one minibatch (tier S with eligibility), see eprop.cu.
@@ -1613,8 +1733,9 @@ int launch_eprop_forward(const EpropLaunch& e, cudaStream_t st) {
   a.elig = e.elig; a.fires = e.fires; a.gamma = e.gamma; a.trace_decay = e.trace_decay;
   a.psi_hist = e.psi_hist; a.psi_T = e.psi_T;
   a.raster = e.raster;
-  if (e.mode == MODE_SORT) return launch_tier_s_kernel<MODE_SORT, true>(g, in->B, a, st);
-  return launch_tier_s_kernel<MODE_ATOMIC, true>(g, in->B, a, st);
+  a.sedges = e.sedges;
+  a.sptr = g->sptr;
+  return launch_tier_s<true>(g, in->B, e.mode, a, st);
 }
 
 // Wave size and ring placement of the tier-G kernel for this run.
@@ -1731,6 +1852,12 @@ static int launch_plain(Run* r, FwdArgs a, cudaStream_t st) {
   return SNC_B200_OK;
 }
 
+// Some delivery mode runs this graph on tier S (ATOMIC's bound is the least).
+bool tier_s_possible(const Graph* g) {
+  return tier_s_bytes(g->N, g->ncols, g->R, std::max(1, g->noc), MODE_ATOMIC, false, 1024) <=
+         (size_t)optin_smem();
+}
+
 static bool tier_s_fits(const Graph* g, int mode) {
   return tier_s_bytes(g->N, g->ncols, g->R, std::max(1, g->noc), mode, false, 1024) <=
          (size_t)optin_smem();
@@ -1779,10 +1906,7 @@ static int launch_body(Run* r, const FwdArgs& a, int mode, int path, cudaStream_
 }
 
 static int launch_kernels(Run* r, const FwdArgs& a, int mode, int path, cudaStream_t st) {
-  if (use_tier_s(r, mode, path)) {
-    if (mode == MODE_SORT) return launch_tier_s<MODE_SORT>(r, a, st);
-    return launch_tier_s<MODE_ATOMIC>(r, a, st);
-  }
+  if (use_tier_s(r, mode, path)) return launch_tier_s<false>(r->g, r->in->B, mode, a, st);
   if (path == SNC_B200_PATH_PERSISTENT) {
     const size_t smem = r->gplan_smem;
     if (r->psi_hist || r->fires) {  // e-prop: ATOMIC or SORT delivery

@@ -7,6 +7,8 @@
 //                  neuron block (post / BS): within a block the CSR order stays
 //   gptr    [N+1], groups [G]  (destination block, first gedge) per row segment
 //   ibase   [P+1]  inbox base of every destination block (groups targeting it)
+//   sedges  [S], sptr [N][32]  (graphs whose state can fit one CTA) each row
+//           regrouped by column range, and the segment starts
 // One warp per row: a counting sort over the P <= kMaxBlocks destination
 // blocks in shared memory, made stable by placing the row's edges 32 at a
 // time in order with match.any ranks.
@@ -134,7 +136,60 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_regroup(BuildArgs a) {
   }
 }
 
+// Rows regrouped by column range for the sample-per-CTA kernel: a warp per
+// row, lane r counting range r; the same stable counting sort as k_regroup.
+__global__ void __launch_bounds__(32 * kRowWarps) k_range_group(int N, int nc, const int* row_ptr,
+                                                               const uint8_t* crange, const uint2* edges,
+                                                               uint2* sedges, int* sptr, int* perm) {
+  __shared__ int cnt[kRowWarps][kSRanges];
+  static_assert(kSPtr <= 32, "a lane per range");
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  int* cn = cnt[wl];
+  for (int i = blockIdx.x * kRowWarps + wl; i < N; i += gridDim.x * kRowWarps) {
+    const int rs = row_ptr[i], re = row_ptr[i + 1];
+    if (lane < kSRanges) cn[lane] = 0;
+    __syncwarp();
+    for (int e = rs + lane; e < re; e += 32) atomicAdd(&cn[crange[edge_col(edges[e])]], 1);
+    __syncwarp();
+    const int c = lane < kSRanges ? cn[lane] : 0;
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane < kSRanges) cn[lane] = rs + incl - c;  // next free place of the range
+    if (sptr && lane < kSPtr) sptr[(size_t)i * kSPtr + lane] = rs + incl - c;  // the last: the row's end
+    __syncwarp();
+    for (int e0 = rs; e0 < re; e0 += 32) {
+      const int e = e0 + lane;
+      const bool valid = e < re;
+      const uint2 ed = valid ? edges[e] : make_uint2(0u, 0u);
+      const int r = valid ? crange[edge_col(ed)] : -1 - lane;
+      const unsigned peers = __match_any_sync(0xffffffffu, r);
+      int at = 0;
+      if (valid) at = cn[r] + __popc(peers & below);
+      __syncwarp();
+      if (valid) {
+        sedges[at] = make_uint2(4u * (uint32_t)(edge_delay(ed) * nc + edge_col(ed)), ed.y);
+        if (perm) perm[e] = at;
+        if ((peers & ~(below | (1u << lane))) == 0) cn[r] = at + 1;  // the last of its range
+      }
+      __syncwarp();
+    }
+  }
+}
+
 }  // namespace
+
+int regroup_by_range(const Graph* g, const uint2* edges, uint2* sedges, int* sptr, int* perm) {
+  if (!g->N) return SNC_B200_OK;
+  const unsigned grid = (unsigned)std::max(1, std::min((g->N + kRowWarps - 1) / kRowWarps, g->sm_count * 16));
+  k_range_group<<<grid, 32 * kRowWarps>>>(g->N, g->ncols, g->row_ptr, g->crange, edges, sedges, sptr, perm);
+  SNCB_CUDA(cudaGetLastError());
+  return SNC_B200_OK;
+}
 
 // The build proper: g->row_ptr, g->post and g->col_of are on the device;
 // w, delays and sign are device columns.
@@ -193,6 +248,11 @@ static int build_core(Graph* g, const float* w, const int* delays, const int8_t*
     SNCB_CUDA(cudaGetLastError());
   }
   if ((rc = scan_exclusive(a.icount, g->ibase, P, scan, nullptr))) return rc;
+  if (g->crange) {
+    if ((rc = dev_alloc(&g->sedges, (size_t)m))) return rc;
+    if ((rc = dev_alloc(&g->sptr, (size_t)n * kSPtr))) return rc;
+    if ((rc = regroup_by_range(g, g->edges, g->sedges, g->sptr, nullptr))) return rc;
+  }
   SNCB_CUDA(cudaDeviceSynchronize());
   return SNC_B200_OK;
 }
