@@ -34,28 +34,28 @@ WaitCtl take_wait_ctl(bool consume);
     if (e_ != cudaSuccess) return cuda_fail(e_, #call);  \
   } while (0)
 
+// pool.cu: device memory (current device) and pinned host memory; released
+// blocks are kept for the next allocation, within bounds.  pool_free waits for
+// the device, as cudaFree does.
+int pool_alloc(void** p, size_t n);
+int pool_alloc_host(void** p, size_t n);
+void pool_free(void* p);
+
+template <typename T>
+int dev_alloc(T** d, size_t n) {
+  return pool_alloc(reinterpret_cast<void**>(d), (n ? n : 1) * sizeof(T));
+}
+
 template <typename T>
 int dev_upload(T** d, const T* h, size_t n) {
-  *d = nullptr;
   if (n == 0) n = 1;
-  if (alloc_fault()) { set_error("device allocation failed (injected)"); return SNC_B200_ENOMEM; }
-  SNCB_CUDA(cudaMalloc(reinterpret_cast<void**>(d), n * sizeof(T)));
+  const int rc = dev_alloc(d, n);
+  if (rc) return rc;
   if (h) SNCB_CUDA(cudaMemcpy(*d, h, n * sizeof(T), cudaMemcpyHostToDevice));
   return SNC_B200_OK;
 }
 
-template <typename T>
-int dev_alloc(T** d, size_t n) {
-  *d = nullptr;
-  if (n == 0) n = 1;
-  if (alloc_fault()) { set_error("device allocation failed (injected)"); return SNC_B200_ENOMEM; }
-  SNCB_CUDA(cudaMalloc(reinterpret_cast<void**>(d), n * sizeof(T)));
-  return SNC_B200_OK;
-}
-
-inline void dev_free(void* p) {
-  if (p) cudaFree(p);
-}
+inline void dev_free(void* p) { pool_free(p); }
 
 // Device-resident graph.  Neurons with at least one incoming synapse own a
 // ring column (col_of[j] >= 0, assigned in ascending id order); the delay

@@ -339,11 +339,12 @@ int HostImage::reserve(size_t n) {
   if (n <= cap) return SNC_B200_OK;
   const size_t want = std::max(n, cap + cap / 2);
   if (pinned) {
-    if (p) cudaFreeHost(p);
+    pool_free(p);
     p = nullptr;
     cap = 0;
     void* q = nullptr;
-    SNCB_CUDA(cudaHostAlloc(&q, want, cudaHostAllocDefault));
+    const int rc = pool_alloc_host(&q, want);
+    if (rc) return rc;
     p = static_cast<unsigned char*>(q);
   } else {
     vec.resize(want);
@@ -354,7 +355,7 @@ int HostImage::reserve(size_t n) {
 }
 
 void HostImage::release() {
-  if (pinned && p) cudaFreeHost(p);
+  if (pinned) pool_free(p);
   vec.clear();
   vec.shrink_to_fit();
   p = nullptr;
@@ -365,14 +366,14 @@ int DevBuf::reserve(size_t n) {
   if (n <= cap) return SNC_B200_OK;
   const size_t want = std::max(n, cap + cap / 2);
   release();
-  if (alloc_fault()) { set_error("device allocation failed (injected)"); return SNC_B200_ENOMEM; }
-  SNCB_CUDA(cudaMalloc(&p, want));
+  const int rc = pool_alloc(&p, want);
+  if (rc) return rc;
   cap = want;
   return SNC_B200_OK;
 }
 
 void DevBuf::release() {
-  if (p) cudaFree(p);
+  pool_free(p);
   p = nullptr;
   cap = 0;
 }
