@@ -494,7 +494,8 @@ int snc_b200_connectome_graph(const snc_b200_connectome* c, snc_b200_graph** out
  *   forward:  v = decay*v + sum_e w_e s_pre(t - d_e) + ext; s = H(v - thr)
  *             (smooth != 0: s = x / (1 + slope |x|)); v = v * (1 - s).
  *             Saves spike_bits [T][N][ceil(B/32)] and v_saved: with
- *             ckpt_every = K > 0, v after every K-th step ([ceil(T/K)][N][B]),
+ *             ckpt_every = K > 0, v after every K-th step and the last
+ *             ([ceil(T/K)][N][B]),
  *             with K = 0 the pre-reset potential of every step ([T][N][B]).
  *   backward: fast-sigmoid surrogate 1 / (1 + slope |x|)^2; grad_w [S] is
  *             overwritten, grad_ext may be NULL.  Recomputes each K-step
