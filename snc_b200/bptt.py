@@ -299,9 +299,10 @@ class SpikingLM(nn.Module):
         return self._core
 
     def forward(self, x):  # [B, T] token ids -> logits [B, T, vocab]
-        B, T = x.shape
-        ext = self.embed(x).transpose(0, 1)                       # [T, B, H]
+        # time outermost throughout, as the core wants it: only the token ids and
+        # the logits change layout, not the hidden activity or its gradients
+        ext = self.embed(x.t())                                   # [T, B, H]
         s = spiking_core(self.w_rec, ext, self.core(), self.thr, self.decay, self.slope,
                          self.ckpt_every)
         r = leaky_scan(s, self.ro_decay)                          # [T, B, H]
-        return self.readout(r.transpose(0, 1))
+        return self.readout(r).transpose(0, 1).contiguous()
