@@ -106,7 +106,8 @@ void free_graph(Graph* g) {
                   (void*)g->out_ch, (void*)g->role, (void*)g->channel, (void*)g->colbase,
                   (void*)g->gedges, (void*)g->gptr, (void*)g->groups, (void*)g->ibase,
                   (void*)g->chan_ptr, (void*)g->chan_ids, (void*)g->ro_rank, (void*)g->ro_chan,
-                  (void*)g->sedges, (void*)g->sptr, (void*)g->crange})
+                  (void*)g->sl[0].sedges, (void*)g->sl[0].sptr, (void*)g->sl[0].range, (void*)g->sl[0].col,
+                  (void*)g->sl[1].sedges, (void*)g->sl[1].sptr, (void*)g->sl[1].range, (void*)g->sl[1].col})
     dev_free(p);
 }
 
@@ -142,6 +143,43 @@ unsigned long long graph_hash_view(const snc_graph_view* v) {
   words(v->sign, n);
   words(v->channel, 4 * n);
   return h;
+}
+
+// Fewest synapses for which a cluster per sample pays: below, a step is bound
+// by its barriers and L2 trips, which a cluster lengthens.  Four samples of
+// recurrent nets, one CTA / four a sample: 57 k synapses 2.7 / 3.3 us a step,
+// 86 k 4.2 / 4.0, 128 k 5.5 / 4.9, 197 k 7.2 / 5.8.
+constexpr int kSClusterEdges = 80000;
+
+// Columns and column ranges of a sample-per-CTA layout (SLayout): within each
+// part the columns by descending in-degree, each to the range with the least so
+// far (first of equals), so hub columns spread over the ranges.
+static int setup_s_layout(const Graph* g, SLayout* L, int cl, const int* indeg) {
+  const int n = g->N;
+  L->cl = cl;
+  std::vector<uint8_t> range((size_t)std::max(1, g->ncols));
+  std::vector<int> col((size_t)std::max(1, n), -1), ids;
+  for (int p = 0; p < cl; ++p) {
+    ids.clear();
+    for (int i = 0; i < n; ++i)
+      if (indeg[i] > 0 && (i >> 5) % cl == p) {
+        col[i] = (int)ids.size();
+        ids.push_back(i);
+      }
+    L->ncols = std::max(L->ncols, (int)ids.size());
+    std::stable_sort(ids.begin(), ids.end(), [&](int x, int y) { return indeg[x] > indeg[y]; });
+    long long load[kSRanges] = {};
+    for (int i : ids) {
+      int r = 0;
+      for (int k = 1; k < kSRanges; ++k)
+        if (load[k] < load[r]) r = k;
+      range[g->col_of_h[i]] = (uint8_t)(p * kSPtr + r);
+      load[r] += indeg[i];
+    }
+  }
+  int rc;
+  if ((rc = dev_upload(&L->range, range.data(), range.size()))) return rc;
+  return dev_upload(&L->col, col.data(), col.size());
 }
 
 // The per-neuron tables of a graph on the host (O(N) work) from its sizes,
@@ -214,25 +252,11 @@ int setup_tables(Graph* g, int n, int m, int max_delay, const int32_t* row_ptr,
     const long long lg = (long long)std::log2(std::max(1, n)) * 64 + (long long)std::log2(std::max(1, m));
     g->signature = (lg << 16) ^ ((long long)(g->fanin_cv * 4) << 8) ^ (long long)g->R;
   }
-  // column ranges of about equal in-degree for the sample-per-CTA kernel: the
-  // columns by descending in-degree, each to the range with the least so far
-  // (first of equals), so hub columns spread over the ranges
-  std::vector<uint8_t> crange;
+  int rc;
   if (tier_s_possible(g)) {
-    crange.resize((size_t)std::max(1, nc));
-    std::vector<int> ids;
-    ids.reserve((size_t)nc);
-    for (int i = 0; i < n; ++i)
-      if (indeg[i] > 0) ids.push_back(i);
-    std::stable_sort(ids.begin(), ids.end(), [&](int x, int y) { return indeg[x] > indeg[y]; });
-    long long load[kSRanges] = {};
-    for (int i : ids) {
-      int r = 0;
-      for (int k = 1; k < kSRanges; ++k)
-        if (load[k] < load[r]) r = k;
-      crange[g->col_of_h[i]] = (uint8_t)r;
-      load[r] += indeg[i];
-    }
+    if ((rc = setup_s_layout(g, &g->sl[0], 1, indeg))) return rc;
+    if (n <= kSCluster * 1024 && m >= kSClusterEdges && (rc = setup_s_layout(g, &g->sl[1], kSCluster, indeg)))
+      return rc;
   }
   std::vector<uint8_t> role(role_v, role_v + n);
   std::vector<int> channel(channel_v, channel_v + n);
@@ -244,10 +268,8 @@ int setup_tables(Graph* g, int n, int m, int max_delay, const int32_t* row_ptr,
       ro_chan.push_back(out_ch[i]);
     }
   g->n_ro = (int)ro_chan.size();
-  int rc;
   if ((rc = dev_upload(&g->col_of, g->col_of_h.data(), (size_t)n))) return rc;
   if ((rc = dev_upload(&g->out_ch, out_ch.data(), (size_t)n))) return rc;
-  if (!crange.empty() && (rc = dev_upload(&g->crange, crange.data(), crange.size()))) return rc;
   if ((rc = dev_upload(&g->role, role.data(), role.size()))) return rc;
   if ((rc = dev_upload(&g->channel, channel.data(), channel.size()))) return rc;
   if ((rc = dev_upload(&g->colbase, colbase.data(), colbase.size()))) return rc;

@@ -55,6 +55,7 @@ struct snc_b200_eprop {
   // sample-per-CTA kernel, by destination block in grid mode (one sample's
   // state does not fit one CTA's shared memory: the all-SM kernel)
   bool grid = false;
+  const sncb::SLayout* layout = nullptr;  // of gedges, unless grid
   int* gperm = nullptr;           // [S] CSR edge -> its regrouped position
   uint2* gedges = nullptr;        // [S+2]
   sncb::Run* run = nullptr;
@@ -317,9 +318,10 @@ static int create_session(snc_b200_eprop* s, const Graph* g, const snc_lif* lif,
     s->grid = tier_s_smem_bytes(g, mode, true) > optin;
   }
   if (!s->grid) {
+    s->layout = &tier_s_layout_of(g, max_batch, cfg->mode == SNC_B200_MODE_SORT ? SNC_B200_MODE_SORT : SNC_B200_MODE_ATOMIC);
     if ((rc = dev_alloc(&s->gperm, (size_t)S))) return rc;
     if ((rc = dev_alloc(&s->gedges, (size_t)S + 2))) return rc;
-    if ((rc = regroup_by_range(g, s->edges, s->gedges, nullptr, s->gperm))) return rc;
+    if ((rc = regroup_by_range(g, *s->layout, s->edges, s->gedges, nullptr, s->gperm))) return rc;
     SNCB_CUDA(cudaDeviceSynchronize());
   } else {
     // the stable regroup of every row by destination block, as the graph's
@@ -387,6 +389,7 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
     set_error("e-prop batch: bad sample count, steps or labels");
     return SNC_B200_EINVAL;
   }
+  DevBuf inline_edges;
   Inputs in;
   int rc = upload_inputs(g, ev, n_ev, B, steps, false, &in);
   if (rc) { free_inputs(&in); return rc; }
@@ -450,6 +453,16 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
     e.in = &in;
     e.edges = s->edges;
     e.sedges = s->gedges;
+    e.layout = s->layout;
+    if (e.elig && e.layout->cl > 1) {
+      // the eligibility accumulated in the forward needs a whole sample in one
+      // CTA: this minibatch's edges in that layout
+      rc = inline_edges.reserve((size_t)std::max(1, S) * sizeof(uint2));
+      if (!rc) rc = regroup_by_range(g, g->sl[0], s->edges, static_cast<uint2*>(inline_edges.p), nullptr, nullptr);
+      ok = rc == SNC_B200_OK;
+      e.sedges = static_cast<uint2*>(inline_edges.p);
+      e.layout = &g->sl[0];
+    }
     e.counts = s->counts;
     e.spikes = s->spikes;
     e.events = s->events;
@@ -466,7 +479,7 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
     e.mode = s->cfg.mode == SNC_B200_MODE_SORT ? SNC_B200_MODE_SORT : SNC_B200_MODE_ATOMIC;
     e.err = s->err;
     e.ctl = s->ctl;
-    rc = launch_eprop_forward(e, st);
+    if (ok) rc = launch_eprop_forward(e, st);
     ok = rc == SNC_B200_OK;
   }
   if (ok) {

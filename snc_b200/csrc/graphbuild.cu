@@ -7,8 +7,8 @@
 //                  neuron block (post / BS): within a block the CSR order stays
 //   gptr    [N+1], groups [G]  (destination block, first gedge) per row segment
 //   ibase   [P+1]  inbox base of every destination block (groups targeting it)
-//   sedges  [S], sptr [N][32]  (graphs whose state can fit one CTA) each row
-//           regrouped by column range, and the segment starts
+//   sl      (graphs whose state can fit one CTA) each row regrouped by column
+//           range for the sample-per-CTA kernel (SLayout)
 // One warp per row: a counting sort over the P <= kMaxBlocks destination
 // blocks in shared memory, made stable by placing the row's edges 32 at a
 // time in order with match.any ranks.
@@ -136,43 +136,53 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_regroup(BuildArgs a) {
   }
 }
 
-// Rows regrouped by column range for the sample-per-CTA kernel: a warp per
-// row, lane r counting range r; the same stable counting sort as k_regroup.
+// Rows regrouped by (part, column range) for the sample-per-CTA kernel: a warp
+// per row, the same stable counting sort as k_regroup over CL * kSPtr bins (the
+// last bin of a part stays empty: its start is the part's end).
+template <int CL>
 __global__ void __launch_bounds__(32 * kRowWarps) k_range_group(int N, int nc, const int* row_ptr,
-                                                               const uint8_t* crange, const uint2* edges,
-                                                               uint2* sedges, int* sptr, int* perm) {
-  __shared__ int cnt[kRowWarps][kSRanges];
-  static_assert(kSPtr <= 32, "a lane per range");
+                                                               const uint8_t* range, const int* col_of_col,
+                                                               const uint2* edges, uint2* sedges, int* sptr,
+                                                               int* perm) {
+  static_assert(kSPtr == 32, "a lane per range");
+  __shared__ int cnt[kRowWarps][CL * kSPtr];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
   int* cn = cnt[wl];
   for (int i = blockIdx.x * kRowWarps + wl; i < N; i += gridDim.x * kRowWarps) {
     const int rs = row_ptr[i], re = row_ptr[i + 1];
-    if (lane < kSRanges) cn[lane] = 0;
-    __syncwarp();
-    for (int e = rs + lane; e < re; e += 32) atomicAdd(&cn[crange[edge_col(edges[e])]], 1);
-    __syncwarp();
-    const int c = lane < kSRanges ? cn[lane] : 0;
-    int incl = c;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
+    for (int p = 0; p < CL; ++p) cn[p * kSPtr + lane] = 0;
+    __syncwarp();
+    for (int e = rs + lane; e < re; e += 32) atomicAdd(&cn[range[edge_col(edges[e])]], 1);
+    __syncwarp();
+    int base = rs;
+#pragma unroll
+    for (int p = 0; p < CL; ++p) {
+      const int c = cn[p * kSPtr + lane];
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      cn[p * kSPtr + lane] = base + incl - c;  // next free place of the range
+      if (sptr) sptr[((size_t)i * CL + p) * kSPtr + lane] = base + incl - c;
+      base += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane < kSRanges) cn[lane] = rs + incl - c;  // next free place of the range
-    if (sptr && lane < kSPtr) sptr[(size_t)i * kSPtr + lane] = rs + incl - c;  // the last: the row's end
     __syncwarp();
     for (int e0 = rs; e0 < re; e0 += 32) {
       const int e = e0 + lane;
       const bool valid = e < re;
       const uint2 ed = valid ? edges[e] : make_uint2(0u, 0u);
-      const int r = valid ? crange[edge_col(ed)] : -1 - lane;
+      const int r = valid ? range[edge_col(ed)] : -1 - lane;
       const unsigned peers = __match_any_sync(0xffffffffu, r);
       int at = 0;
       if (valid) at = cn[r] + __popc(peers & below);
       __syncwarp();
       if (valid) {
-        sedges[at] = make_uint2(4u * (uint32_t)(edge_delay(ed) * nc + edge_col(ed)), ed.y);
+        const int c = col_of_col[edge_col(ed)];
+        sedges[at] = make_uint2(4u * (uint32_t)(edge_delay(ed) * nc + c), ed.y);
         if (perm) perm[e] = at;
         if ((peers & ~(below | (1u << lane))) == 0) cn[r] = at + 1;  // the last of its range
       }
@@ -181,12 +191,27 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_range_group(int N, int nc, c
   }
 }
 
+// Column within its part of every column of the graph.
+__global__ void k_part_cols(int N, const int* col_of, const int* col, int* out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
+    if (col_of[i] >= 0) out[col_of[i]] = col[i];
+}
+
 }  // namespace
 
-int regroup_by_range(const Graph* g, const uint2* edges, uint2* sedges, int* sptr, int* perm) {
+int regroup_by_range(const Graph* g, const SLayout& L, const uint2* edges, uint2* sedges, int* sptr, int* perm) {
   if (!g->N) return SNC_B200_OK;
+  DevBuf pc;
+  int rc = pc.reserve((size_t)std::max(1, g->ncols) * 4);
+  if (rc) return rc;
+  int* cols = static_cast<int*>(pc.p);
   const unsigned grid = (unsigned)std::max(1, std::min((g->N + kRowWarps - 1) / kRowWarps, g->sm_count * 16));
-  k_range_group<<<grid, 32 * kRowWarps>>>(g->N, g->ncols, g->row_ptr, g->crange, edges, sedges, sptr, perm);
+  k_part_cols<<<grid, 256>>>(g->N, g->col_of, L.col, cols);
+  if (L.cl > 1)
+    k_range_group<kSCluster><<<grid, 32 * kRowWarps>>>(g->N, L.ncols, g->row_ptr, L.range, cols, edges, sedges,
+                                                       sptr, perm);
+  else
+    k_range_group<1><<<grid, 32 * kRowWarps>>>(g->N, L.ncols, g->row_ptr, L.range, cols, edges, sedges, sptr, perm);
   SNCB_CUDA(cudaGetLastError());
   return SNC_B200_OK;
 }
@@ -248,10 +273,13 @@ static int build_core(Graph* g, const float* w, const int* delays, const int8_t*
     SNCB_CUDA(cudaGetLastError());
   }
   if ((rc = scan_exclusive(a.icount, g->ibase, P, scan, nullptr))) return rc;
-  if (g->crange) {
-    if ((rc = dev_alloc(&g->sedges, (size_t)m))) return rc;
-    if ((rc = dev_alloc(&g->sptr, (size_t)n * kSPtr))) return rc;
-    if ((rc = regroup_by_range(g, g->edges, g->sedges, g->sptr, nullptr))) return rc;
+  for (SLayout& L : g->sl) {
+    if (!L.range) continue;
+    uint2* se = nullptr;
+    if ((rc = dev_alloc(&L.sptr, (size_t)n * L.cl * kSPtr))) return rc;
+    if ((rc = dev_alloc(&se, (size_t)m))) return rc;
+    L.sedges = se;
+    if ((rc = regroup_by_range(g, L, g->edges, se, L.sptr, nullptr))) return rc;
   }
   SNCB_CUDA(cudaDeviceSynchronize());
   return SNC_B200_OK;

@@ -66,6 +66,22 @@ struct OneShot;
 // Column ranges of the sample-per-CTA kernel (one per warp but the last of its
 // CTA) and the entries of a row of sptr: the segment starts, the row's end.
 constexpr int kSRanges = 31, kSPtr = kSRanges + 1;
+constexpr int kSCluster = 4;  // CTAs of a cluster that shares one sample
+
+// Edges for the sample-per-CTA kernel of cl CTAs a sample.  Part p of cl holds
+// the neurons of the 32-neuron words p, p + cl, ... and their ring columns,
+// numbered from 0 within the part (col; ncols: the most of any part).  Each
+// row's edges are stably regrouped by (part, column range of the part):
+// sedges (4 (delay * ncols + column), weight); sptr: the start of every (row,
+// part, range) segment and the end of the part's last.  range: part * kSPtr +
+// range of each column of the graph.
+struct SLayout {
+  int cl = 1, ncols = 0;
+  uint2* sedges = nullptr;   // [S]
+  int* sptr = nullptr;       // [N][cl][kSPtr]
+  uint8_t* range = nullptr;  // [graph columns]
+  int* col = nullptr;        // [N] column within the part or -1
+};
 
 struct Graph {
   int N = 0, S = 0, R = 0, ncols = 0, noc = 0, nic = 0, max_delay = 1;
@@ -96,13 +112,9 @@ struct Graph {
   // targeting b) descriptors per step, stored from ibase[b].
   int G = 0;
   int* ibase = nullptr;     // [P+1]
-  // graphs whose state can fit one CTA: each row's edges stably regrouped by
-  // column range (4 (delay * ncols + column), weight), and the start of every
-  // row's segment of every range, then the row's end; crange: the range of
-  // each column
-  uint2* sedges = nullptr;     // [S]
-  int* sptr = nullptr;         // [N][kSPtr]
-  uint8_t* crange = nullptr;   // [ncols]
+  // graphs whose state can fit one CTA: the sample-per-CTA layout, and that of
+  // a cluster per sample where it pays (sedges null: none)
+  SLayout sl[2];
   // leaky readout units (OUTPUT neurons with a channel, ascending id): rank of
   // each neuron among them or -1, and each rank's channel
   int n_ro = 0;
@@ -239,7 +251,8 @@ struct EpropLaunch {
   const Graph* g = nullptr;
   const Inputs* in = nullptr;
   const uint2* edges = nullptr;  // packed edges carrying the trainer's weights
-  const uint2* sedges = nullptr; // the same regrouped by column range
+  const uint2* sedges = nullptr; // the same in the layout's order
+  const SLayout* layout = nullptr;
   int* counts = nullptr;         // [B][max(1,noc)]
   unsigned long long* spikes = nullptr;
   unsigned long long* events = nullptr;
@@ -290,10 +303,10 @@ int build_graph_device(const snc_graph_view* v, Graph* g);
 // The same from columns already on the device (g->row_ptr, g->post and
 // g->col_of set; weights, delays and per-neuron signs as device arrays).
 int build_graph_device_cols(Graph* g, const float* w, const int* delays, const int8_t* sign);
-// Edges in CSR order (packed as g->edges) regrouped by column range into
-// sedges [S]; sptr [N][kSPtr] and perm [S] (CSR edge -> its place in
-// sedges) are written when given.  In stream order on the legacy stream.
-int regroup_by_range(const Graph* g, const uint2* edges, uint2* sedges, int* sptr, int* perm);
+// Edges in CSR order (packed as g->edges) regrouped for layout L into sedges
+// [S]; sptr and perm [S] (CSR edge -> its place in sedges) are written when
+// given.  In stream order on the legacy stream.
+int regroup_by_range(const Graph* g, const SLayout& L, const uint2* edges, uint2* sedges, int* sptr, int* perm);
 // The schedule of a batch encoded on the device from its features.
 int encode_inputs(const Graph* g, int enc, const float* features, int C, int B, const int32_t* steps,
                   float gain, float max_rate, float threshold, uint64_t seed, Inputs* in);
@@ -321,6 +334,7 @@ int launch_eprop_forward(const EpropLaunch& e, cudaStream_t stream);
 int launch_run(Run* r, const snc_lif* lif, int mode, int path, cudaStream_t stream);
 int tier_s_smem_bytes(const Graph* g, int mode, bool eprop);
 bool tier_s_possible(const Graph* g);  // N, ncols, R and noc set
+const SLayout& tier_s_layout_of(const Graph* g, int B, int mode);
 // AUTO resolution: the autotuned choice cached for this graph and batch (mode,
 // path and launch shape: shape[4] = tier, threads, wave, ring_smem), else a
 // default rule (shape automatic).

@@ -22,14 +22,20 @@ CASES = {
     "long_segments": (600, 300, 8, 0.9, 4, 1, 6, 0.6),            # more than 1024 events of a warp's batch
     "tags_per_warp": (150, 560, 8, 0.06, 68, 2, 80, 0.1),         # too many cells for a tag each
     "brimful": (40, 330, 10, 0.1, 149, 2, 160, 0.2),              # no room for scratch
+    "cluster": (500, 700, 9, 0.12, 9, 3, 15, 0.1),                # 80,000 synapses and more
+    "cluster_large": (2400, 600, 9, 0.06, 5, 2, 8, 0.15),
     "hubs": (700, 3, 2, 1.0, 2, 2, 10, 0.5),                      # hundreds of events a cell
 }
 
 
+# few samples run a cluster of CTAs each, many a CTA each
+@pytest.mark.parametrize("many", [False, True])
 @pytest.mark.parametrize("mode", [R.MODE_SORT, R.MODE_ATOMIC])
 @pytest.mark.parametrize("name", sorted(CASES))
-def test_layout(name, mode):
+def test_layout(name, mode, many):
     n_in, n_hid, n_out, p, max_delay, samples, steps, rate = CASES[name]
+    if many:
+        samples, steps = 40, max(2, steps // 4)
     g = W.random_graph(5, n_in=n_in, n_hid=n_hid, n_out=n_out, p=p, max_delay=max_delay)
     scale = min(1.0, 8.0 / max(1.0, g.num_synapses / g.num_neurons))
     g.weights[:] = np.rint(g.weights * scale * 4096.0) / 4096.0
