@@ -45,12 +45,33 @@ __device__ __forceinline__ void red_release_add_u32(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Block-wide exclusive scan of one int per thread (blockDim a multiple of 32,
+// Threads that work together: a whole CTA, or some of its warps that meet at a
+// named barrier of their own (slot: the group's number in the CTA).
+struct CtaGroup {
+  static constexpr int kGroups = 1;
+  __device__ __forceinline__ int tid() const { return threadIdx.x; }
+  __device__ __forceinline__ int size() const { return blockDim.x; }
+  __device__ __forceinline__ int slot() const { return 0; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+struct WarpGroup {
+  static constexpr int kGroups = 4;
+  int t, n, g;
+  __device__ __forceinline__ int tid() const { return t; }
+  __device__ __forceinline__ int size() const { return n; }
+  __device__ __forceinline__ int slot() const { return g; }
+  __device__ __forceinline__ void sync() const {
+    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(n) : "memory");
+  }
+};
+
+// Exclusive scan of one int per thread of a group (a multiple of 32 threads,
 // at most 1024).  scratch: >= 33 ints of shared memory.  Returns this
-// thread's exclusive prefix and writes the block total to *total.
-__device__ __forceinline__ int block_exclusive_scan(int x, int* scratch, int* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
+// thread's exclusive prefix and writes the group's total to *total.
+template <class G>
+__device__ __forceinline__ int group_exclusive_scan(const G& grp, int x, int* scratch, int* total) {
+  const int lane = grp.tid() & 31, warp = grp.tid() >> 5;
+  const int nw = grp.size() >> 5;
   int incl = x;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -58,7 +79,7 @@ __device__ __forceinline__ int block_exclusive_scan(int x, int* scratch, int* to
     if (lane >= o) incl += y;
   }
   if (lane == 31) scratch[warp] = incl;
-  __syncthreads();
+  grp.sync();
   if (warp == 0) {
     int s = lane < nw ? scratch[lane] : 0;
     int si = s;
@@ -70,11 +91,16 @@ __device__ __forceinline__ int block_exclusive_scan(int x, int* scratch, int* to
     if (lane < nw) scratch[lane] = si - s;
     if (lane == 31) scratch[32] = si;
   }
-  __syncthreads();
+  grp.sync();
   const int res = scratch[warp] + incl - x;
   *total = scratch[32];
-  __syncthreads();
+  grp.sync();
   return res;
+}
+
+// The same over the whole CTA.
+__device__ __forceinline__ int block_exclusive_scan(int x, int* scratch, int* total) {
+  return group_exclusive_scan(CtaGroup(), x, scratch, total);
 }
 
 // Block-wide sum of one 64-bit value per thread; result valid in all threads.
@@ -218,12 +244,13 @@ namespace sncb {
 // Ordered compaction of one flag per thread with warp ballot / popc: returns
 // the number of flagged threads before this one in thread order, writes the
 // block total to *total and this warp's ballot to *mask.  scratch >= 33 ints.
-__device__ __forceinline__ int ballot_compact(int flag, int* scratch, int* total, unsigned* mask) {
+template <class G>
+__device__ __forceinline__ int ballot_compact(const G& grp, int flag, int* scratch, int* total, unsigned* mask) {
   const unsigned m = __ballot_sync(0xffffffffu, flag);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
+  const int lane = grp.tid() & 31, warp = grp.tid() >> 5;
+  const int nw = grp.size() >> 5;
   if (lane == 0) scratch[warp] = __popc(m);
-  __syncthreads();
+  grp.sync();
   if (warp == 0) {
     const int c = lane < nw ? scratch[lane] : 0;
     int incl = c;
@@ -235,11 +262,11 @@ __device__ __forceinline__ int ballot_compact(int flag, int* scratch, int* total
     if (lane < nw) scratch[lane] = incl - c;
     if (lane == 31) scratch[32] = incl;
   }
-  __syncthreads();
+  grp.sync();
   const int pos = scratch[warp] + __popc(m & ((1u << lane) - 1u));
   *total = scratch[32];
   *mask = m;
-  __syncthreads();
+  grp.sync();
   return pos;
 }
 
@@ -247,21 +274,18 @@ __device__ __forceinline__ int ballot_compact(int flag, int* scratch, int* total
 // per-warp counts itself, and the caller alternates between two 32-int
 // buffers (a buffer is written again only two calls later, after every
 // thread has passed the barrier of the call in between).  blockDim <= 1024.
-__device__ __forceinline__ int ballot_compact_1(int flag, int* buf, int* total, unsigned* mask) {
+template <class G>
+__device__ __forceinline__ int ballot_compact_1(const G& grp, int flag, int* buf, int* total, unsigned* mask) {
   const unsigned m = __ballot_sync(0xffffffffu, flag);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
+  const int lane = grp.tid() & 31, warp = grp.tid() >> 5;
+  const int nw = grp.size() >> 5;
   if (lane == 0) buf[warp] = __popc(m);
-  __syncthreads();
-  const int c = lane < nw ? buf[lane] : 0;
-  int incl = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const int before = __shfl_sync(0xffffffffu, incl - c, warp);
-  *total = __shfl_sync(0xffffffffu, incl, 31);
+  grp.sync();
+  // (flagged in earlier warps, flagged in all) in one sum: at most 1024 each
+  const unsigned c = lane < nw ? (unsigned)buf[lane] : 0u;
+  const unsigned both = __reduce_add_sync(0xffffffffu, (lane < warp ? c : 0u) | (c << 16));
+  const int before = (int)(both & 0xffffu);
+  *total = (int)(both >> 16);
   *mask = m;
   return before + __popc(m & ((1u << lane) - 1u));
 }

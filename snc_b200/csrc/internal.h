@@ -213,6 +213,7 @@ struct Run {
   int* inbox_cnt = nullptr;             // [Bw][2][P]
   bool gplan_rsm = false;    // tier G keeps ring slices in shared memory
   size_t gplan_smem = 0;
+  int gplan_groups = 1, gplan_gthreads = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.f;
   int used_mode = -1, used_path = -1;
