@@ -305,6 +305,13 @@ static int upload_graph(const snc_graph_view* v, Graph* g) {
 void free_run(Run* r) {
   if (!r) return;
   if (r->gexec) cudaGraphExecDestroy(r->gexec);
+  if (r->outs) {
+    dev_free(r->outs);
+    r->counts = nullptr;
+    r->spikes = r->events = nullptr;
+    r->err = nullptr;
+    r->ctl = nullptr;
+  }
   for (void* p : {(void*)r->counts, (void*)r->spikes, (void*)r->events, (void*)r->raster,
                   (void*)r->vfinal, (void*)r->err, (void*)r->ctl, (void*)r->v, (void*)r->refr,
                   (void*)r->ring, (void*)r->fired, (void*)r->fired_cnt, (void*)r->inbox,
@@ -315,6 +322,26 @@ void free_run(Run* r) {
   if (r->own_stream) cudaStreamDestroy(r->own_stream);
 }
 
+int place_outputs(Run* r, int B, int noc) {
+  const size_t Bn = (size_t)std::max(1, B);
+  const size_t o_ev = kOutsSpikes + 8 * Bn, o_cnt = o_ev + 8 * Bn;
+  r->outs_bytes = o_cnt + 4 * Bn * std::max(1, noc);
+  if (r->outs_bytes > r->outs_cap) {
+    dev_free(r->outs);
+    r->outs = nullptr;
+    r->outs_cap = 0;
+    const int rc = dev_alloc(&r->outs, r->outs_bytes);
+    if (rc) return rc;
+    r->outs_cap = r->outs_bytes;
+  }
+  r->err = reinterpret_cast<int*>(r->outs);
+  r->ctl = reinterpret_cast<unsigned*>(r->outs + 16);
+  r->spikes = reinterpret_cast<unsigned long long*>(r->outs + kOutsSpikes);
+  r->events = reinterpret_cast<unsigned long long*>(r->outs + o_ev);
+  r->counts = reinterpret_cast<int*>(r->outs + o_cnt);
+  return SNC_B200_OK;
+}
+
 static int create_run(const Graph* g, const Inputs* in, int flags, Run* r) {
   r->g = g;
   r->in = in;
@@ -322,15 +349,11 @@ static int create_run(const Graph* g, const Inputs* in, int flags, Run* r) {
   r->W = (g->N + 31) / 32;
   const size_t B = (size_t)std::max(1, in->B);
   int rc;
-  if ((rc = dev_alloc(&r->counts, B * std::max(1, g->noc)))) return rc;
-  if ((rc = dev_alloc(&r->spikes, B))) return rc;
-  if ((rc = dev_alloc(&r->events, B))) return rc;
+  if ((rc = place_outputs(r, in->B, g->noc))) return rc;
   if (flags & SNC_B200_RUN_RASTER)
     if ((rc = dev_alloc(&r->raster, (size_t)std::max<long long>(1, in->raster_words)))) return rc;
   if (flags & SNC_B200_RUN_VFINAL)
     if ((rc = dev_alloc(&r->vfinal, B * std::max(1, g->N)))) return rc;
-  if ((rc = dev_alloc(&r->err, 1))) return rc;
-  if ((rc = dev_alloc(&r->ctl, 4))) return rc;
   SNCB_CUDA(cudaEventCreate(&r->ev0));
   SNCB_CUDA(cudaEventCreate(&r->ev1));
   return SNC_B200_OK;
@@ -346,27 +369,33 @@ int fetch_run(Run* r, float* logits, int64_t* spikes, int64_t* events, uint32_t*
   r->last_ms = ms;
   const int B = in->B, noc = std::max(1, g->noc);
   const bool ro = logits && r->ro_decay >= 0.f && r->ro_logits && B > 0;
-  // pinned block: err, schedule err | spikes [B] | events [B] | counts [B][noc] | readout [B][noc]
+  // pinned block: err, ... | spikes [B] | events [B] | counts [B][noc] |
+  // schedule err | readout [B][noc]; the first four as the device block
   const size_t Bn = (size_t)std::max(0, B);
-  const size_t o_sp = 8, o_ev = o_sp + 8 * Bn, o_cnt = o_ev + 8 * Bn;
-  const size_t o_lg = o_cnt + 4 * Bn * noc, total = o_lg + (ro ? 4 * Bn * noc : 0);
+  const size_t o_sp = kOutsSpikes, o_ev = o_sp + 8 * std::max<size_t>(1, Bn), o_cnt = o_ev + 8 * std::max<size_t>(1, Bn);
+  const size_t o_se = o_cnt + 4 * std::max<size_t>(1, Bn) * noc, o_lg = o_se + 8;
+  const size_t total = o_lg + (ro ? 4 * Bn * noc : 0);
   int rc;
   if ((rc = r->fetch_img.reserve(total))) return rc;
   unsigned char* h = r->fetch_img.p;
   std::memset(h, 0, 8);
+  std::memset(h + o_se, 0, 8);
   const cudaStream_t s0 = cudaStreamPerThread;
-  SNCB_CUDA(cudaMemcpyAsync(h, r->err, 4, cudaMemcpyDeviceToHost, s0));
-  if (d_sched_err) SNCB_CUDA(cudaMemcpyAsync(h + 4, d_sched_err, 4, cudaMemcpyDeviceToHost, s0));
+  if (r->outs) SNCB_CUDA(cudaMemcpyAsync(h, r->outs, r->outs_bytes, cudaMemcpyDeviceToHost, s0));
+  else SNCB_CUDA(cudaMemcpyAsync(h, r->err, 4, cudaMemcpyDeviceToHost, s0));
+  if (d_sched_err) SNCB_CUDA(cudaMemcpyAsync(h + o_se, d_sched_err, 4, cudaMemcpyDeviceToHost, s0));
   if (B > 0) {
-    SNCB_CUDA(cudaMemcpyAsync(h + o_sp, r->spikes, 8 * Bn, cudaMemcpyDeviceToHost, s0));
-    SNCB_CUDA(cudaMemcpyAsync(h + o_ev, r->events, 8 * Bn, cudaMemcpyDeviceToHost, s0));
-    SNCB_CUDA(cudaMemcpyAsync(h + o_cnt, r->counts, 4 * Bn * noc, cudaMemcpyDeviceToHost, s0));
+    if (!r->outs) {
+      SNCB_CUDA(cudaMemcpyAsync(h + o_sp, r->spikes, 8 * Bn, cudaMemcpyDeviceToHost, s0));
+      SNCB_CUDA(cudaMemcpyAsync(h + o_ev, r->events, 8 * Bn, cudaMemcpyDeviceToHost, s0));
+      SNCB_CUDA(cudaMemcpyAsync(h + o_cnt, r->counts, 4 * Bn * noc, cudaMemcpyDeviceToHost, s0));
+    }
     if (ro) SNCB_CUDA(cudaMemcpyAsync(h + o_lg, r->ro_logits, 4 * Bn * noc, cudaMemcpyDeviceToHost, s0));
   }
   SNCB_CUDA(cudaStreamSynchronize(s0));
   int err = 0;
   std::memcpy(&err, h, 4);
-  if (sched_err) std::memcpy(sched_err, h + 4, 4);
+  if (sched_err) std::memcpy(sched_err, h + o_se, 4);
   const int* counts = reinterpret_cast<const int*>(h + o_cnt);
   const unsigned long long* sp = reinterpret_cast<const unsigned long long*>(h + o_sp);
   const unsigned long long* evn = reinterpret_cast<const unsigned long long*>(h + o_ev);

@@ -31,7 +31,11 @@ struct snc_b200_eprop {
   float* delta = nullptr;                // [max_batch][oc]
   float* L = nullptr;                    // [max_batch][N]
   int* labels = nullptr;                 // [max_batch]
-  int* steps = nullptr;                  // [max_batch]
+  // err, ctl, spikes, events and counts of a minibatch in one block, cleared and
+  // read back (through img) with one operation each
+  unsigned char* outs = nullptr;
+  size_t outs_bytes = 0;
+  sncb::HostImage img{true};
   unsigned long long* spikes = nullptr;  // [max_batch]
   unsigned long long* events = nullptr;  // [max_batch]
   unsigned long long* fires = nullptr;   // [N]
@@ -225,9 +229,7 @@ __global__ void k_elig_col(int B, int N, int S, int nc, int G, const int* cptr, 
 
 static void free_session(snc_b200_eprop* s) {
   for (void* p : {(void*)s->edges, (void*)s->bmat, (void*)s->internal_row, (void*)s->elig,
-                  (void*)s->counts, (void*)s->delta, (void*)s->L, (void*)s->labels,
-                  (void*)s->steps, (void*)s->spikes, (void*)s->events, (void*)s->fires,
-                  (void*)s->err, (void*)s->ctl})
+                  (void*)s->outs, (void*)s->delta, (void*)s->L, (void*)s->labels, (void*)s->fires})
     dev_free(p);
   if (s->ev0) cudaEventDestroy(s->ev0);
   if (s->ev1) cudaEventDestroy(s->ev1);
@@ -296,16 +298,19 @@ static int create_session(snc_b200_eprop* s, const Graph* g, const snc_lif* lif,
   if ((rc = dev_upload(&s->internal_row, irow.data(), (size_t)N))) return rc;
   const size_t B = (size_t)max_batch;
   if ((rc = dev_alloc(&s->elig, B * std::max(1, S)))) return rc;
-  if ((rc = dev_alloc(&s->counts, B * s->oc))) return rc;
   if ((rc = dev_alloc(&s->delta, B * s->oc))) return rc;
   if ((rc = dev_alloc(&s->L, B * std::max(1, N)))) return rc;
   if ((rc = dev_alloc(&s->labels, B))) return rc;
-  if ((rc = dev_alloc(&s->steps, B))) return rc;
-  if ((rc = dev_alloc(&s->spikes, B))) return rc;
-  if ((rc = dev_alloc(&s->events, B))) return rc;
+  const size_t o_ev = kOutsSpikes + 8 * B, o_cnt = o_ev + 8 * B;
+  s->outs_bytes = o_cnt + 4 * B * s->oc;
+  if ((rc = dev_alloc(&s->outs, s->outs_bytes))) return rc;
+  if ((rc = s->img.reserve(s->outs_bytes))) return rc;
+  s->err = reinterpret_cast<int*>(s->outs);
+  s->ctl = reinterpret_cast<unsigned*>(s->outs + 16);
+  s->spikes = reinterpret_cast<unsigned long long*>(s->outs + kOutsSpikes);
+  s->events = reinterpret_cast<unsigned long long*>(s->outs + o_ev);
+  s->counts = reinterpret_cast<int*>(s->outs + o_cnt);
   if ((rc = dev_alloc(&s->fires, (size_t)std::max(1, N)))) return rc;
-  if ((rc = dev_alloc(&s->err, 1))) return rc;
-  if ((rc = dev_alloc(&s->ctl, 4))) return rc;
   SNCB_CUDA(cudaMemset(s->fires, 0, (size_t)std::max(1, N) * sizeof(unsigned long long)));
   SNCB_CUDA(cudaEventCreate(&s->ev0));
   SNCB_CUDA(cudaEventCreate(&s->ev1));
@@ -399,11 +404,7 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
   auto chk = [&](cudaError_t e, const char* what) {
     if (ok && e != cudaSuccess) { rc = cuda_fail(e, what); ok = false; }
   };
-  chk(cudaMemsetAsync(s->counts, 0, (size_t)B * oc * sizeof(int), st), "memset counts");
-  chk(cudaMemsetAsync(s->spikes, 0, (size_t)B * 8, st), "memset spikes");
-  chk(cudaMemsetAsync(s->events, 0, (size_t)B * 8, st), "memset events");
-  chk(cudaMemsetAsync(s->ctl, 0, 16, st), "memset ctl");
-  chk(cudaMemsetAsync(s->err, 0, 4, st), "memset err");
+  chk(cudaMemsetAsync(s->outs, 0, s->outs_bytes, st), "memset outputs");
   // deferred eligibility when the psi history of this minibatch fits its budget
   const int W = (N + 31) / 32;
   const size_t psi_bytes = (size_t)B * std::max(1, g->ncols) * std::max(1, in.Tmax) * sizeof(float);
@@ -426,10 +427,7 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
     }
   }
   if (train && !deferred) chk(cudaMemsetAsync(s->elig, 0, (size_t)B * S * sizeof(float), st), "memset elig");
-  if (train) {
-    chk(cudaMemcpyAsync(s->labels, labels, (size_t)B * 4, cudaMemcpyHostToDevice, st), "labels");
-    chk(cudaMemcpyAsync(s->steps, steps, (size_t)B * 4, cudaMemcpyHostToDevice, st), "steps");
-  }
+  if (train) chk(cudaMemcpyAsync(s->labels, labels, (size_t)B * 4, cudaMemcpyHostToDevice, st), "labels");
   chk(cudaEventRecord(s->ev0, st), "event");
   if (ok && s->grid) {
     // the all-SM kernel with the trainer's weights, recording psi and the
@@ -508,10 +506,10 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
     k_learning_signal<<<grid_of((long long)B * N), 256, 0, st>>>(
         B, N, oc, s->cfg.train_hidden, g->role, g->channel, s->internal_row, s->bmat, s->delta, s->L);
     if (train == 2)
-      k_gradient<<<grid_of(S), 256, 0, st>>>(S, N, B, g->post, s->steps, s->L, s->elig, grad);
+      k_gradient<<<grid_of(S), 256, 0, st>>>(S, N, B, g->post, in.steps, s->L, s->elig, grad);
     else
       k_apply<<<grid_of(S), 256, 0, st>>>(S, N, B, uniform ? 1 : 0, s->cfg.lr, lr_over_T,
-                                          s->cfg.w_max, g->post, s->steps, s->L, s->elig, s->edges);
+                                          s->cfg.w_max, g->post, in.steps, s->L, s->elig, s->edges);
     chk(cudaGetLastError(), "e-prop update kernels");
     if (train == 1 && ok) {
       const int r2 = sync_gedges(s, st);
@@ -519,15 +517,15 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
     }
   }
   chk(cudaEventRecord(s->ev1, st), "event");
-  chk(cudaEventSynchronize(s->ev1), "synchronize");
+  chk(cudaMemcpyAsync(s->img.p, s->outs, s->outs_bytes, cudaMemcpyDeviceToHost, st), "results");
+  chk(cudaStreamSynchronize(st), "synchronize");
   if (ok) {
-    std::vector<int> cnt((size_t)B * oc);
-    std::vector<unsigned long long> sp(B), en(B);
-    chk(cudaMemcpy(cnt.data(), s->counts, cnt.size() * 4, cudaMemcpyDeviceToHost), "counts");
-    chk(cudaMemcpy(sp.data(), s->spikes, (size_t)B * 8, cudaMemcpyDeviceToHost), "spikes");
-    chk(cudaMemcpy(en.data(), s->events, (size_t)B * 8, cudaMemcpyDeviceToHost), "events");
-    int err = 0;
-    chk(cudaMemcpy(&err, s->err, 4, cudaMemcpyDeviceToHost), "err");
+    const unsigned char* h = s->img.p;
+    auto at = [&](const void* d) { return h + (static_cast<const unsigned char*>(d) - s->outs); };
+    const int* cnt = reinterpret_cast<const int*>(at(s->counts));
+    const unsigned long long* sp = reinterpret_cast<const unsigned long long*>(at(s->spikes));
+    const unsigned long long* en = reinterpret_cast<const unsigned long long*>(at(s->events));
+    const int err = *reinterpret_cast<const int*>(at(s->err));
     if (ok && counts_out)
       for (int b = 0; b < B; ++b)
         for (int c = 0; c < g->noc; ++c) counts_out[(size_t)b * g->noc + c] = (float)cnt[(size_t)b * oc + c];

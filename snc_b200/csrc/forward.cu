@@ -2141,11 +2141,15 @@ int launch_run(Run* r, const snc_lif* lif, int mode, int path, cudaStream_t st) 
     if (!r->own_stream) SNCB_CUDA(cudaStreamCreate(&r->own_stream));
     st = r->own_stream;
   }
-  SNCB_CUDA(cudaMemsetAsync(r->counts, 0, B * std::max(1, g->noc) * sizeof(int), st));
-  SNCB_CUDA(cudaMemsetAsync(r->spikes, 0, B * sizeof(unsigned long long), st));
-  SNCB_CUDA(cudaMemsetAsync(r->events, 0, B * sizeof(unsigned long long), st));
-  SNCB_CUDA(cudaMemsetAsync(r->ctl, 0, 4 * sizeof(unsigned), st));
-  SNCB_CUDA(cudaMemsetAsync(r->err, 0, sizeof(int), st));
+  if (r->outs) {
+    SNCB_CUDA(cudaMemsetAsync(r->outs, 0, r->outs_bytes, st));
+  } else {
+    SNCB_CUDA(cudaMemsetAsync(r->counts, 0, B * std::max(1, g->noc) * sizeof(int), st));
+    SNCB_CUDA(cudaMemsetAsync(r->spikes, 0, B * sizeof(unsigned long long), st));
+    SNCB_CUDA(cudaMemsetAsync(r->events, 0, B * sizeof(unsigned long long), st));
+    SNCB_CUDA(cudaMemsetAsync(r->ctl, 0, 4 * sizeof(unsigned), st));
+    SNCB_CUDA(cudaMemsetAsync(r->err, 0, sizeof(int), st));
+  }
   if (r->inbox_cnt)
     SNCB_CUDA(cudaMemsetAsync(r->inbox_cnt, 0, (size_t)r->Bw_cap * 2 * g->P * sizeof(int), st));
   if ((r->flags & SNC_B200_RUN_RASTER) && in->raster_words)

@@ -202,6 +202,10 @@ struct Run {
   // control
   int* err = nullptr;
   unsigned* ctl = nullptr;  // [0] barrier counter, [1] work-queue counter
+  // err, ctl, spikes, events and counts in one block (null: separate arrays),
+  // cleared and read back with one operation each
+  unsigned char* outs = nullptr;
+  size_t outs_cap = 0, outs_bytes = 0;
   // grid-path state (one wave of Bw samples in lockstep)
   int Bw = 0, Bw_cap = 0;
   float* v = nullptr;
@@ -276,7 +280,6 @@ struct OneShot {
   DevBuf keep, work;  // the schedule and the builder's work arrays
   Inputs in;
   Run run;
-  int B_cap = 0;
   cudaStream_t stream = nullptr;
 };
 
@@ -322,6 +325,11 @@ int oneshot_forward(const Graph* g, const snc_input_event* ev, size_t n_ev, int 
 void free_oneshot(const Graph* g);
 
 // api.cu
+// Places a run's error word, control words and per-sample results for B
+// samples in its one block, grown on demand (o_spikes: their offset; events
+// and counts follow).
+constexpr size_t kOutsSpikes = 32;
+int place_outputs(Run* r, int B, int noc);
 // Waits for the run and copies its results out.  d_sched_err, when given,
 // is the schedule builder's overflow word, read in the same batch of copies
 // into *sched_err.

@@ -774,21 +774,8 @@ int oneshot_forward(const Graph* g, const snc_input_event* ev, size_t n_ev, int 
     r.W = (g->N + 31) / 32;
     SNCB_CUDA(cudaEventCreate(&r.ev0));
     SNCB_CUDA(cudaEventCreate(&r.ev1));
-    if ((rc = dev_alloc(&r.err, 1))) return rc;
-    if ((rc = dev_alloc(&r.ctl, 4))) return rc;
   }
-  const int Bc = std::max(1, B);
-  if (Bc > ws->B_cap) {
-    for (void* p : {(void*)r.counts, (void*)r.spikes, (void*)r.events}) dev_free(p);
-    r.counts = nullptr;
-    r.spikes = nullptr;
-    r.events = nullptr;
-    ws->B_cap = 0;
-    if ((rc = dev_alloc(&r.counts, (size_t)Bc * std::max(1, g->noc)))) return rc;
-    if ((rc = dev_alloc(&r.spikes, (size_t)Bc))) return rc;
-    if ((rc = dev_alloc(&r.events, (size_t)Bc))) return rc;
-    ws->B_cap = Bc;
-  }
+  if ((rc = place_outputs(&r, B, g->noc))) return rc;
   if ((rc = launch_run(&r, lif, mode, path, ws->stream))) return rc;
   int err = 0;
   rc = fetch_run(&r, logits, spikes, events_out, nullptr, nullptr, stats, in.d_err, &err);
