@@ -186,8 +186,12 @@ __global__ void k_raster_t(int B, int N, int W, int TW, const int* steps, const 
 // incoming synapses of one column): the column's psi history is read once
 // per 32 steps (one gather of 32 steps, then broadcast by shuffles; the
 // history is step-major so that the forward writes each step's values for
-// all columns contiguously) and each
-// lane's pre spikes come 32 steps to a word from the transposed raster.
+// all columns contiguously) and each lane's pre spikes come 32 steps to a word
+// from the transposed raster.
+// FIN: a finite surrogate scale, so that psi is finite and a step of zero trace
+// adds a zero of either sign, which no sum that began at +0 shows: it needs no
+// test then (32 samples of 1000 steps, 144,000 synapses: 929 -> 791 us).
+template <bool FIN>
 __global__ void k_elig_col(int B, int N, int S, int nc, int G, const int* cptr, const int2* cin,
                            const int* gptr, const int* steps, const uint32_t* rt, int TW,
                            const float* psi, int psi_T, float decay, float* elig) {
@@ -214,7 +218,7 @@ __global__ void k_elig_col(int B, int N, int S, int nc, int G, const int* cptr, 
         const float p = __shfl_sync(0xffffffffu, pv, u);
         const float dt = __fmul_rn(decay, tr);
         tr = (word >> u) & 1u ? __fadd_rn(dt, c1) : dt;
-        if (tr != 0.f) acc = __fadd_rn(acc, __fmul_rn(p, tr));
+        if (FIN || tr != 0.f) acc = __fadd_rn(acc, __fmul_rn(p, tr));
       };
       if (T - t0 >= 32) {
 #pragma unroll
@@ -492,7 +496,7 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
           B, N, W, TW, in.steps, in.raster_off, static_cast<const uint32_t*>(s->raster.p), rt);
       const long long warps = (long long)B * s->n_groups;
       if (warps > 0)
-        k_elig_col<<<(int)std::max(1ll, std::min((warps + 7) / 8, (long long)sms * 16)), 256, 0, st>>>(
+        (std::isfinite(s->cfg.surrogate_scale) ? k_elig_col<true> : k_elig_col<false>)<<<(int)std::max(1ll, std::min((warps + 7) / 8, (long long)sms * 16)), 256, 0, st>>>(
             B, N, S, std::max(1, g->ncols), s->n_groups, s->cptr, s->cin, s->gptr, in.steps, rt, TW,
             static_cast<const float*>(s->psi_hist.p), std::max(1, in.Tmax), s->cfg.trace_decay, s->elig);
       chk(cudaGetLastError(), "deferred eligibility");
