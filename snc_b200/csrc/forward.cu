@@ -542,12 +542,13 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
   const uint2* __restrict__ sed = a.sedges;
 
   float vr[KN ? KN : 1];
-  int rf[KN ? KN : 1], colr[KN ? KN : 1];
+  int rf[KN ? KN : 1], colr[KN ? KN : 1], colg[EP && CL > 1 && KN ? KN : 1];  // colg: in the graph
   unsigned outm = 0;  // bit c: the neuron is an output with a channel
 #pragma unroll
   for (int c = 0; c < nch; ++c) {
     const int j = 32 * word_of(c) + lane;
     if (KN) colr[KN ? c : 0] = j < N ? a.s_col[j] : -1;
+    if (EP && CL > 1) colg[EP && CL > 1 && KN ? c : 0] = j < N ? a.col_of[j] : -1;
     if (j < N && a.out_ch[j] >= 0) outm |= 1u << c;
   }
   const unsigned rom = a.ro_on ? outm : 0u;  // bit c: a leaky readout unit
@@ -654,7 +655,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
               if (thr > 0.f && thr != 1.f) dd = __fdiv_rn(dd, thr);  // x / 1 = x
               const float ps = dd < 1.f ? __fmul_rn(a.gamma, __fsub_rn(1.f, dd)) : 0.f;
               if (inl) psi[col] = ps;
-              if (psi_t) psi_t[CL > 1 ? a.col_of[j] : col] = ps;
+              if (psi_t) psi_t[EP && CL > 1 ? colg[EP && CL > 1 && KN ? c : 0] : col] = ps;
             }
             if (inl)
               tr[j] = __fadd_rn(__fmul_rn(a.trace_decay, tr[j]),
