@@ -46,6 +46,7 @@
 struct snc_b200_bptt {
   int N = 0, S = 0, D = 1, R = 2, sm_count = 0;
   int max_deg = 0;     // largest in- or out-degree
+  bool even = false;   // runs of 32 neurons have about the same number of edges
   int resident = 1;    // allow resident launches
   int *row_ptr = nullptr, *out_post = nullptr, *out_d = nullptr;
   int *col_ptr = nullptr, *in_pre = nullptr, *in_d = nullptr, *in_eidx = nullptr;
@@ -81,6 +82,7 @@ struct BpArgs {
   int Bp;              // samples of a padded row (SL * VB * 32)
   float* ring;         // resident backward: [R][N][Bp] future gradients
   int res_cap;         // resident launches: edges per direction staged per warp
+  int even;            // resident launches: items in order, not round the CTAs
   unsigned long long wait_ns;  // grid-barrier wait bound (0: the default)
   unsigned stall;              // injected arrivals that never come (failure tests)
 };
@@ -534,7 +536,12 @@ __global__ void __launch_bounds__(kBpThreads, kBpMinBlocks<KB>) k_bptt_backward(
 // per edge and passed through shared memory.
 //
 // Items go round the CTAs (item i to CTA i mod grid), so that neurons without
-// synapses in one direction share an SM with others.
+// synapses in one direction share an SM with others; where every run of 32
+// neurons has about the same number of edges (a.even) they are dealt in
+// order, and neighbours of a net with local synapses find rows that they share
+// in L1.  4096 neurons on a ring, 64 samples: backward 3487 -> 3240 us,
+// forward 1057 -> 1023; the layers of 784, 512 and 512 neurons in order would
+// take 1869 and 740 us instead of 1705 and 594.
 
 template <int VB>
 struct VecOf;
@@ -662,7 +669,7 @@ template <int VB, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) k_res_forward(BpArgs a) {
   extern __shared__ __align__(16) float sm_all[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int item = warp * gridDim.x + blockIdx.x;
+  const int item = a.even ? (int)(blockIdx.x * (blockDim.x >> 5)) + warp : warp * (int)gridDim.x + (int)blockIdx.x;
   const bool on = item < a.N * a.SL;
   const int j = on ? item % a.N : 0, sl = on ? item / a.N : 0;
   const int N = a.N, B = a.B, b0 = sl * 32 * VB + lane;
@@ -738,7 +745,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_backward(BpArgs a) {
   typedef typename VecOf<VB>::T Vec;
   extern __shared__ __align__(16) float sm_all[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int item = warp * gridDim.x + blockIdx.x;
+  const int item = a.even ? (int)(blockIdx.x * (blockDim.x >> 5)) + warp : warp * (int)gridDim.x + (int)blockIdx.x;
   const bool on = item < a.N * a.SL;
   const int j = on ? item % a.N : 0, sl = on ? item / a.N : 0;
   const int N = a.N, B = a.B, T = a.T, R = a.R, K = a.K, cap = a.res_cap;
@@ -1088,6 +1095,7 @@ static BpArgs forward_args(const snc_b200_bptt* h, const float* w, const float* 
   a.in_pre = h->in_pre; a.in_d = h->in_d; a.in_eidx = h->in_eidx;
   a.w = w; a.ext = ext; a.spikes = spikes; a.bits = spike_bits; a.vsaved = v_saved;
   a.res_cap = res_cap(h);
+  a.even = h->even;
   pick_slices(a, h->sm_count);
   const WaitCtl wc = take_wait_ctl(true);
   a.wait_ns = wc.ns;
@@ -1238,6 +1246,14 @@ int snc_b200_bptt_create(int32_t N, int32_t S, const int32_t* row_ptr, const int
   for (int j = 0; j < N; ++j)
     h->max_deg = std::max({h->max_deg, col_ptr[j + 1], row_ptr[j + 1] - row_ptr[j]});
   for (int j = 0; j < N; ++j) col_ptr[j + 1] += col_ptr[j];
+  // (a quarter above the mean: a random net of 64 synapses a neuron stays
+  // within a tenth; a layer without synapses in one direction is at 3/2)
+  h->even = true;
+  for (int j = 0; j < N && h->even; j += 32) {
+    const int k = std::min(N, j + 32);
+    const double edges = (double)(col_ptr[k] - col_ptr[j]) + (row_ptr[k] - row_ptr[j]);
+    h->even = edges * N <= 1.25 * 2.0 * S * 32;
+  }
   std::vector<int> fill(col_ptr.begin(), col_ptr.end() - 1);
   for (int i = 0; i < N; ++i)
     for (int e = row_ptr[i]; e < row_ptr[i + 1]; ++e) {
@@ -1329,6 +1345,7 @@ int snc_b200_bptt_backward(snc_b200_bptt* h, const float* w, const float* ext, i
   a.gspk = grad_spikes; a.gw = grad_w; a.gext = grad_ext;
   a.ctl = h->ctl; a.err = h->err;
   a.res_cap = res_cap(h);
+  a.even = h->even;
   pick_slices(a, h->sm_count);
   const bool rs = rs_fits(a, h->sm_count);
   // the resident form keeps its state in registers and pads its rows
