@@ -398,6 +398,12 @@ int snc_b200_eprop_create(const snc_b200_graph* g, const snc_lif* lif, const snc
  * fits one CTA (the sample-per-CTA kernel), SNC_B200_PATH_PERSISTENT when it
  * does not (the all-SM kernel on a destination-grouped copy of the weights). */
 int snc_b200_eprop_path(const snc_b200_eprop* s);
+/* Most bytes of device memory the surrogate history of one training minibatch
+ * may take (samples x neurons with incoming synapses x steps x 4; 0: the
+ * default, 2 GiB).  A minibatch beyond it accumulates its eligibility step by
+ * step in the forward instead, with the same result; on the all-SM kernel it is
+ * refused (SNC_B200_EUNSUPPORTED).  No reference counterpart. */
+int snc_b200_eprop_set_history_limit(snc_b200_eprop* s, uint64_t bytes);
 int snc_b200_eprop_release(snc_b200_eprop* s);                    /* cudatrain::destroy */
 int snc_b200_eprop_set_weights(snc_b200_eprop* s, const float* w); /* [S] */
 int snc_b200_eprop_get_weights(snc_b200_eprop* s, float* w);       /* [S] */

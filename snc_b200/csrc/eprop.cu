@@ -18,6 +18,10 @@
 #include "device_common.cuh"
 #include "internal.h"
 
+// Most bytes the psi history of one minibatch may take by default; beyond it
+// the eligibility is accumulated inside the forward instead.
+static constexpr size_t kPsiHistMax = size_t(2) << 30;
+
 struct snc_b200_eprop {
   const sncb::Graph* g = nullptr;
   snc_lif lif{};
@@ -47,6 +51,7 @@ struct snc_b200_eprop {
   // deferred eligibility: the forward records psi per ring column and step
   // and the spike raster; k_raster_t and k_elig_col then build E from them
   sncb::DevBuf psi_hist, raster, raster_t;
+  size_t psi_max = kPsiHistMax;
   // incoming synapses of every ring column: (edge, pre) pairs grouped by
   // column (cin[cptr[c] .. cptr[c+1])), and the prefix of their 32-synapse
   // groups (gptr) -- the deferred eligibility's work items
@@ -145,10 +150,6 @@ static int sync_gedges(snc_b200_eprop* s, cudaStream_t st) {
   SNCB_CUDA(cudaGetLastError());
   return SNC_B200_OK;
 }
-
-// Most bytes the psi history of one minibatch may take; beyond it the
-// eligibility is accumulated inside the forward instead.
-constexpr size_t kPsiHistMax = size_t(2) << 30;
 
 // The spike raster ([t][word] bits, raster_off per sample) transposed to
 // one run of time bits per neuron: rt[b][i][w] bit u = fired_i(32 w + u)
@@ -412,7 +413,7 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
   // deferred eligibility when the psi history of this minibatch fits its budget
   const int W = (N + 31) / 32;
   const size_t psi_bytes = (size_t)B * std::max(1, g->ncols) * std::max(1, in.Tmax) * sizeof(float);
-  const bool deferred = train && psi_bytes <= kPsiHistMax;
+  const bool deferred = train && psi_bytes <= s->psi_max;
   if (train && s->grid && !deferred) {
     free_inputs(&in);
     set_error("e-prop: the minibatch's psi history exceeds its budget on the grid path; use fewer samples or steps");
@@ -456,9 +457,11 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
     e.edges = s->edges;
     e.sedges = s->gedges;
     e.layout = s->layout;
+    e.elig = train && !deferred ? s->elig : nullptr;
     if (e.elig && e.layout->cl > 1) {
       // the eligibility accumulated in the forward needs a whole sample in one
-      // CTA: this minibatch's edges in that layout
+      // CTA (the surrogates lie in its shared memory by the graph's column):
+      // this minibatch's edges in that layout
       rc = inline_edges.reserve((size_t)std::max(1, S) * sizeof(uint2));
       if (!rc) rc = regroup_by_range(g, g->sl[0], s->edges, static_cast<uint2*>(inline_edges.p), nullptr, nullptr);
       ok = rc == SNC_B200_OK;
@@ -468,7 +471,6 @@ static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, 
     e.counts = s->counts;
     e.spikes = s->spikes;
     e.events = s->events;
-    e.elig = train && !deferred ? s->elig : nullptr;
     e.fires = train ? s->fires : nullptr;
     if (deferred) {
       e.psi_hist = static_cast<float*>(s->psi_hist.p);
@@ -574,6 +576,12 @@ int snc_b200_eprop_create(const snc_b200_graph* g, const snc_lif* lif, const snc
   int rc = create_session(s, static_cast<const Graph*>(g), lif, cfg, max_batch, weights, feedback);
   if (rc) { free_session(s); delete s; return rc; }
   *out = s;
+  return SNC_B200_OK;
+}
+
+int snc_b200_eprop_set_history_limit(snc_b200_eprop* s, uint64_t bytes) {
+  if (!s) { set_error("null session"); return SNC_B200_EINVAL; }
+  s->psi_max = bytes ? (size_t)bytes : kPsiHistMax;
   return SNC_B200_OK;
 }
 

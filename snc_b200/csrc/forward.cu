@@ -1810,6 +1810,11 @@ static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, cons
     return kn == 1 ? k_tier_s<1, EP, kSOrdered, 1> : kn == 2 ? k_tier_s<2, EP, kSOrdered, 1>
            : kn == 4 ? k_tier_s<4, EP, kSOrdered, 1> : k_tier_s<0, EP, kSOrdered, 1>;
   };
+  if (L.cl > 1 && EP && a.elig) {
+    // its CTAs hold the surrogates of their own columns only
+    set_error("tier S: eligibility in the forward needs a whole sample in one CTA");
+    return SNC_B200_EUNSUPPORTED;
+  }
   cudaFuncAttributes fa{};
   SNCB_CUDA(cudaFuncGetAttributes(&fa, pick(2, kSOrdered)));
   const size_t budget = (size_t)optin_smem() - fa.sharedSizeBytes;

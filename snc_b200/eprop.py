@@ -93,6 +93,12 @@ class CudaTrainSession:
         does not fit one CTA's shared memory)."""
         return lib().snc_b200_eprop_path(self.h) == _lib.PATH_PERSISTENT
 
+    def set_history_limit(self, nbytes: int) -> None:
+        """Most bytes the surrogate history of a training minibatch may take
+        (0: the default, 2 GiB); beyond it the eligibility is accumulated in
+        the forward, with the same result."""
+        check(lib().snc_b200_eprop_set_history_limit(self.h, int(nbytes)), "eprop_set_history_limit")
+
     def get_weights(self) -> np.ndarray:
         w = np.zeros(self.g.num_synapses, np.float32)
         check(lib().snc_b200_eprop_get_weights(self.h, ptr(w)), "eprop_get_weights")
