@@ -1428,7 +1428,10 @@ __device__ void phase_b(const G& grp, const FwdArgs& a, const GSmem& sm, int* sc
   }
   grp.sync();
   const int cnt = s_cnt;
-  if (cnt == 0) return;
+  if (cnt == 0) {
+    if (tail_sync) grp.sync();  // the next sample's count goes to the same word
+    return;
+  }
   if (cnt <= (MODE == MODE_SORT ? kFastDesc : 32) &&
       phase_b_fast<MODE, RSM>(grp, a, sm, k, s0, cb0, cnt, spec, spec2, tail_sync))
     return;
