@@ -177,6 +177,10 @@ static int setup_s_layout(const Graph* g, SLayout* L, int cl, const int* indeg) 
       load[r] += indeg[i];
     }
   }
+  if (cl > 1 && !tier_s_cluster_fits(g, *L)) {  // (the columns may all lie in one part)
+    *L = SLayout();
+    return SNC_B200_OK;
+  }
   int rc;
   if ((rc = dev_upload(&L->range, range.data(), range.size()))) return rc;
   return dev_upload(&L->col, col.data(), col.size());

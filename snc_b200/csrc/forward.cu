@@ -1822,7 +1822,7 @@ static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, cons
   SNCB_CUDA(cudaFuncGetAttributes(&fa, pick(2, kSOrdered)));
   const size_t budget = (size_t)optin_smem() - fa.sharedSizeBytes;
   const SPlan p = tier_s_layout(g, L, a.noc, EP && a.elig, mode, budget);
-  if (L.cl > 1 && p.del != kSOrdered) {  // (a quarter of a state that fits one CTA)
+  if (L.cl > 1 && p.del != kSOrdered) {  // (no such layout is built: tier_s_cluster_fits)
     set_error("tier S: a cluster's part does not fit on an SM");
     return SNC_B200_EUNSUPPORTED;
   }
@@ -2029,6 +2029,23 @@ static int launch_plain(Run* r, FwdArgs a, cudaStream_t st) {
 bool tier_s_possible(const Graph* g) {
   return tier_s_bytes(g->N, g->ncols, g->R, std::max(1, g->noc), MODE_ATOMIC, false, 1024) <=
          (size_t)optin_smem();
+}
+
+// Each of a cluster's CTAs has room for the ordered delivery.  Its part holds
+// the columns of every kSCluster-th word of 32 neurons, a quarter of them when
+// they are spread, all of them when those words are the ones with synapses.
+bool tier_s_cluster_fits(const Graph* g, const SLayout& L) {
+  size_t fixed = 0;
+  for (const void* f : {(const void*)k_tier_s<1, false, kSOrdered, kSCluster>,
+                        (const void*)k_tier_s<1, true, kSOrdered, kSCluster>}) {
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    fixed = std::max(fixed, (size_t)fa.sharedSizeBytes);
+  }
+  return tier_s_layout(g, L, std::max(1, g->noc), false, MODE_SORT, (size_t)optin_smem() - fixed).del == kSOrdered;
 }
 
 static bool tier_s_fits(const Graph* g, int mode) {
