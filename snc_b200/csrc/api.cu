@@ -177,9 +177,12 @@ static int setup_s_layout(const Graph* g, SLayout* L, int cl, const int* indeg) 
       load[r] += indeg[i];
     }
   }
-  if (cl > 1 && !tier_s_cluster_fits(g, *L)) {  // (the columns may all lie in one part)
-    *L = SLayout();
-    return SNC_B200_OK;
+  if (cl > 1) {
+    L->max_samples = tier_s_clusters(g, *L);
+    if (!L->max_samples) {  // (the columns may all lie in one part)
+      *L = SLayout();
+      return SNC_B200_OK;
+    }
   }
   int rc;
   if ((rc = dev_upload(&L->range, range.data(), range.size()))) return rc;

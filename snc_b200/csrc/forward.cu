@@ -491,7 +491,7 @@ __device__ __forceinline__ void stage_row(const int* __restrict__ sptr, int j, i
 // time by a search per event and ordered through cell bitmaps and a hash table;
 // ATOMIC 4.1 us, 6.0 with the rows of a warp's list fetched one after another;
 // a 1050-neuron net with 90 short rows a step 4.3 us, 5.2 before.  Clusters of
-// four: 5.8 us for up to 37 samples.  Slower: 16 ranges and warps (too few in
+// four: 5.8 us for up to 33 samples.  Slower: 16 ranges and warps (too few in
 // flight), owners that add one row's segment at a time without a conflict check
 // (130 cycles a row for the chain), match.any for the conflicts (100 cycles a
 // group), edges requested 4 or 8 groups ahead in registers (they share
@@ -1800,6 +1800,23 @@ static SPlan tier_s_layout(const Graph* g, const SLayout& L, int noc, bool inl, 
   return p;
 }
 
+// A launch of cl CTAs for each of `samples` samples; attr: one attribute, kept
+// as long as the configuration.
+static cudaLaunchConfig_t s_config(int cl, int samples, size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(cl * samples);
+  cfg.blockDim = dim3(kSThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = cl;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cl > 1 ? 1 : 0;
+  return cfg;
+}
+
 template <bool EP>
 static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, const FwdArgs& a_in, cudaStream_t st) {
   FwdArgs a = a_in;
@@ -1822,7 +1839,7 @@ static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, cons
   SNCB_CUDA(cudaFuncGetAttributes(&fa, pick(2, kSOrdered)));
   const size_t budget = (size_t)optin_smem() - fa.sharedSizeBytes;
   const SPlan p = tier_s_layout(g, L, a.noc, EP && a.elig, mode, budget);
-  if (L.cl > 1 && p.del != kSOrdered) {  // (no such layout is built: tier_s_cluster_fits)
+  if (L.cl > 1 && p.del != kSOrdered) {  // (no such layout is built: tier_s_clusters)
     set_error("tier S: a cluster's part does not fit on an SM");
     return SNC_B200_EUNSUPPORTED;
   }
@@ -1839,28 +1856,22 @@ static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, cons
     set_error("tier S does not fit on an SM");
     return SNC_B200_EUNSUPPORTED;
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(L.cl > 1 ? B * L.cl : std::max(1, std::min(B, per_sm * g->sm_count)));
-  cfg.blockDim = dim3(kSThreads);
-  cfg.dynamicSmemBytes = p.smem;
-  cfg.stream = st;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = L.cl;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = L.cl > 1 ? 1 : 0;
+  const int samples = L.cl > 1 ? B : std::max(1, std::min(B, per_sm * g->sm_count));
+  const cudaLaunchConfig_t cfg = s_config(L.cl, samples, p.smem, st, attr);
   SNCB_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
   return SNC_B200_OK;
 }
 
 // The layout a batch of B samples runs on: ordered delivery on clusters while
-// all of them fit the device at once (ATOMIC is faster in one CTA, 3.8 against
-// 5.8 us a step on the 1744-neuron net).
+// the device holds all of them at once -- fewer than its SMs would make, since
+// a cluster stays within one GPC: 33 of four CTAs on 148 SMs.  34 samples of the
+// 1744-neuron net take a second round, 7.2 us a step against 3.8 for 33 and 4.1
+// in one CTA each.  (ATOMIC is faster in one CTA, 3.8 against 5.8 us a step at a
+// higher rate.)
 const SLayout& tier_s_layout_of(const Graph* g, int B, int mode) {
   const SLayout& c = g->sl[1];
-  return mode == MODE_SORT && c.sedges && (long long)B * c.cl <= g->sm_count ? c : g->sl[0];
+  return mode == MODE_SORT && c.sedges && B <= c.max_samples ? c : g->sl[0];
 }
 
 // e-prop forward of one minibatch (tier S with eligibility), see eprop.cu.
@@ -2031,21 +2042,31 @@ bool tier_s_possible(const Graph* g) {
          (size_t)optin_smem();
 }
 
-// Each of a cluster's CTAs has room for the ordered delivery.  Its part holds
-// the columns of every kSCluster-th word of 32 neurons, a quarter of them when
-// they are spread, all of them when those words are the ones with synapses.
-bool tier_s_cluster_fits(const Graph* g, const SLayout& L) {
-  size_t fixed = 0;
-  for (const void* f : {(const void*)k_tier_s<1, false, kSOrdered, kSCluster>,
-                        (const void*)k_tier_s<1, true, kSOrdered, kSCluster>}) {
+// Clusters of layout L that the device holds at once, 0 if a CTA of one lacks the
+// room for the ordered delivery.  A part holds the columns of every kSCluster-th
+// word of 32 neurons, a quarter of them when they are spread, all of them when
+// those words are the ones with synapses.
+int tier_s_clusters(const Graph* g, const SLayout& L) {
+  int least = 0;
+  void (*const kerns[])(FwdArgs) = {k_tier_s<1, false, kSOrdered, kSCluster>, k_tier_s<1, true, kSOrdered, kSCluster>};
+  for (auto kern : kerns) {
     cudaFuncAttributes fa{};
-    if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
+    int n = 0;
+    bool ok = cudaFuncGetAttributes(&fa, kern) == cudaSuccess;
+    const size_t budget = (size_t)optin_smem() - std::min((size_t)optin_smem(), fa.sharedSizeBytes);
+    const SPlan p = tier_s_layout(g, L, std::max(1, g->noc), false, MODE_SORT, budget);
+    ok = ok && p.del == kSOrdered &&
+         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) == cudaSuccess;
+    if (ok) {
+      cudaLaunchAttribute attr[1];
+      const cudaLaunchConfig_t cfg = s_config(L.cl, g->sm_count, p.smem, nullptr, attr);
+      ok = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess;
     }
-    fixed = std::max(fixed, (size_t)fa.sharedSizeBytes);
+    cudaGetLastError();
+    if (!ok || n < 1) return 0;
+    least = least ? std::min(least, n) : n;
   }
-  return tier_s_layout(g, L, std::max(1, g->noc), false, MODE_SORT, (size_t)optin_smem() - fixed).del == kSOrdered;
+  return least;
 }
 
 static bool tier_s_fits(const Graph* g, int mode) {

@@ -77,6 +77,7 @@ constexpr int kSCluster = 4;  // CTAs of a cluster that shares one sample
 // range of each column of the graph.
 struct SLayout {
   int cl = 1, ncols = 0;
+  int max_samples = 0;       // clusters: as many as the device holds at once
   uint2* sedges = nullptr;   // [S]
   int* sptr = nullptr;       // [N][cl][kSPtr]
   uint8_t* range = nullptr;  // [graph columns]
@@ -343,7 +344,7 @@ int launch_eprop_forward(const EpropLaunch& e, cudaStream_t stream);
 int launch_run(Run* r, const snc_lif* lif, int mode, int path, cudaStream_t stream);
 int tier_s_smem_bytes(const Graph* g, int mode, bool eprop);
 bool tier_s_possible(const Graph* g);  // N, ncols, R and noc set
-bool tier_s_cluster_fits(const Graph* g, const SLayout& L);  // L.cl and L.ncols set as well
+int tier_s_clusters(const Graph* g, const SLayout& L);  // L.cl and L.ncols set as well
 const SLayout& tier_s_layout_of(const Graph* g, int B, int mode);
 // AUTO resolution: the autotuned choice cached for this graph and batch (mode,
 // path and launch shape: shape[4] = tier, threads, wave, ring_smem), else a
