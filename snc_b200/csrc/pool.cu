@@ -10,9 +10,11 @@
 //             device -- the wait cudaFree makes as well -- so no stream of any
 //             thread can still use it; one mutex guards the lists
 //   bounded   at most kKeepDevice bytes per device and kKeepHost pinned bytes
-//             are kept; a block that would exceed them is freed
+//             are kept; a block that would exceed them is freed, and one that
+//             never could be kept is not rounded up to a class
 //   returned  everything kept is freed when the last live block is released
-//             and when an allocation fails (which is then tried again)
+//             and when an allocation fails (which is then tried again, without
+//             the rounding)
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -28,9 +30,12 @@ constexpr size_t kKeepDevice = size_t(256) << 20;
 constexpr size_t kKeepHost = size_t(32) << 20;
 constexpr int kHost = -1;  // "device" of pinned host blocks
 
+size_t keep_limit(int dev) { return dev == kHost ? kKeepHost : kKeepDevice; }
+
 struct Block {
   int dev;
   size_t bytes;
+  bool classed;  // its size is a class, so another allocation can take it
 };
 
 struct Pool {
@@ -46,8 +51,10 @@ Pool& pool() {
   return *p;
 }
 
-// Powers of two up to 1 MiB, then four sizes between each two.
-size_t size_class(size_t n) {
+// Powers of two up to 1 MiB, then four sizes between each two; blocks too large
+// to be kept as they are.
+size_t size_class(size_t n, int dev) {
+  if (n > keep_limit(dev)) return n;
   size_t c = 512;
   while (c < n) c <<= 1;
   if (c > (size_t(1) << 20)) {
@@ -77,7 +84,7 @@ void trim(Pool& q, int dev) {
 }
 
 int take(void** out, size_t n, int dev) {
-  const size_t c = size_class(n);
+  size_t c = size_class(n, dev);
   Pool& q = pool();
   std::lock_guard<std::mutex> lk(q.mu);
   auto& list = q.kept[{dev, c}];
@@ -91,11 +98,12 @@ int take(void** out, size_t n, int dev) {
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
       trim(q, dev);
+      c = n;  // what was asked for is what must fit
       e = raw_alloc(&p, c, dev);
     }
     if (e != cudaSuccess) return cuda_fail(e, dev == kHost ? "cudaHostAlloc" : "cudaMalloc");
   }
-  q.live[p] = Block{dev, c};
+  q.live[p] = Block{dev, c, c == size_class(n, dev)};
   *out = p;
   return SNC_B200_OK;
 }
@@ -133,7 +141,7 @@ void pool_free(void* p) {
   std::lock_guard<std::mutex> lk(q.mu);
   q.live.erase(p);
   size_t& kept = q.kept_bytes[b.dev];
-  if (idle && kept + b.bytes <= (b.dev == kHost ? kKeepHost : kKeepDevice)) {
+  if (idle && b.classed && kept + b.bytes <= keep_limit(b.dev)) {
     q.kept[{b.dev, b.bytes}].push_back(p);
     kept += b.bytes;
   } else {
