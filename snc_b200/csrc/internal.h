@@ -36,7 +36,7 @@ WaitCtl take_wait_ctl(bool consume);
 
 // pool.cu: device memory (current device) and pinned host memory; released
 // blocks are kept for the next allocation, within bounds.  pool_free waits for
-// the device, as cudaFree does.
+// the device, as cudaFree does, and leaves other threads' stream captures alone.
 int pool_alloc(void** p, size_t n);
 int pool_alloc_host(void** p, size_t n);
 void pool_free(void* p);
