@@ -531,9 +531,10 @@ __global__ void __launch_bounds__(kBpThreads, kBpMinBlocks<KB>) k_bptt_backward(
 // synapses of delay 1.  Everything else -- the gather over the other synapses,
 // the weight gradient, the recomputation of a checkpoint segment -- runs
 // between the arrival at a step's barrier and the wait for it.  G lies in a
-// ring of padded rows, read as VB-wide vectors; rows of steps beyond T are
-// zero, so no edge needs a check.  Edge offsets of a step are computed once
-// per edge and passed through shared memory.
+// ring of padded rows, read as VB-wide vectors.  Edge offsets of a step are
+// computed once per edge and passed through shared memory.  Edges that reach
+// beyond T are left out (an infinite weight times a zero gradient would be NaN):
+// only the last steps, as many as the largest delay, look for them.
 //
 // Items go round the CTAs (item i to CTA i mod grid), so that neurons without
 // synapses in one direction share an SM with others; where every run of 32
@@ -795,16 +796,23 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_backward(BpArgs a) {
     for (int k = 0; k < VB; ++k) acc[k] = __fmaf_rn(p.y, reinterpret_cast<const float*>(&x)[k], acc[k]);
   };
   // acc += the gradients of out-edges [e0, e1) at step t, in that order
-  // (base: the step's slot * N)
-  auto gather = [&](int base, int e0, int e1, float (&acc)[VB]) {
+  // (base: the step's slot * N; left: steps from t to the end)
+  constexpr unsigned kBeyond = 0xffffffffu;
+  auto gather = [&](int base, int left, int e0, int e1, float (&acc)[VB]) {
+    const int lim = left < R ? left * N : ring_n;  // orow < lim: within T
     for (int e = e0 + lane; e < e1; e += 32) {
-      int r = base + we.orow[e];
+      const int o = we.orow[e];
+      int r = base + o;
       if (r >= ring_n) r -= ring_n;
-      we.pair[e].x = __uint_as_float((unsigned)r * row_b);
+      we.pair[e].x = __uint_as_float(o < lim ? (unsigned)r * row_b : kBeyond);
     }
     __syncwarp();
     constexpr int U = VB == 4 ? 4 : 8;
     int e = e0;
+    if (lim < ring_n) {
+      for (; e < e1; ++e)
+        if (__float_as_uint(we.pair[e].x) != kBeyond) one(e, acc);
+    }
     for (; e < e1 && (e & 1); ++e) one(e, acc);
     for (; e + U <= e1; e += U) {
       Vec x[U];
@@ -873,7 +881,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_backward(BpArgs a) {
       vp[k] = K == 0 ? (bb + k < B ? a.vsaved[plane + k] : 0.f)
                      : a.seg[((size_t)kp * N + j) * a.Bp + bb + k];
     }
-    gather(base, we.none, we.nout, gs);
+    gather(base, T - t, we.none, we.nout, gs);
   };
   unsigned target = a.stall;
   if (on) prepare(T - 1);
@@ -883,7 +891,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_backward(BpArgs a) {
       float g1[VB];
 #pragma unroll
       for (int k = 0; k < VB; ++k) g1[k] = 0.f;
-      gather(base, 0, we.none, g1);
+      gather(base, T - t, 0, we.none, g1);
       Vec out;
 #pragma unroll
       for (int k = 0; k < VB; ++k) {
@@ -1362,8 +1370,7 @@ int snc_b200_bptt_backward(snc_b200_bptt* h, const float* w, const float* ext, i
   a.stall = wc.stall;
   SNCB_CUDA(cudaMemsetAsync(h->ctl, 0, 16, st));
   SNCB_CUDA(cudaMemsetAsync(h->err, 0, 4, st));
-  if (rs) SNCB_CUDA(cudaMemsetAsync(a.ring, 0, (size_t)h->R * rows * sizeof(float), st));
-  else SNCB_CUDA(cudaMemsetAsync(a.part, 0, (size_t)a.SL * std::max(1, h->S) * sizeof(float), st));
+  if (!rs) SNCB_CUDA(cudaMemsetAsync(a.part, 0, (size_t)a.SL * std::max(1, h->S) * sizeof(float), st));
   if ((rc = launch(false, smooth != 0, a, h->sm_count, st))) return rc;
   if (h->S > 0) {
     k_sum_slices<<<std::min((h->S + 255) / 256, h->sm_count * 8), 256, 0, st>>>(h->S, a.SL, a.part, grad_w);
