@@ -496,7 +496,8 @@ int snc_b200_connectome_graph(const snc_b200_connectome* c, snc_b200_graph** out
  * All tensors are DEVICE pointers, batch innermost: ext / spikes / grads are
  * [T][N][B] fp32, weights [S] in CSR order.  Calls are ordered on `stream`
  * (a cudaStream_t) and return after it has drained; one handle must not be
- * used from two streams at once (it owns the workspaces).
+ * used from two streams at once (it owns the workspaces).  At most 256 samples
+ * (SNC_B200_EUNSUPPORTED beyond).
  *   forward:  v = decay*v + sum_e w_e s_pre(t - d_e) + ext; s = H(v - thr)
  *             (smooth != 0: s = x / (1 + slope |x|)); v = v * (1 - s).
  *             Saves spike_bits [T][N][ceil(B/32)] and v_saved: with

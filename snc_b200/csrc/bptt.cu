@@ -1045,10 +1045,12 @@ static int rs_launch(bool forward, const BpArgs& a, int sm, cudaStream_t st) {
   return SNC_B200_OK;
 }
 
+constexpr int kMaxWords = 8;  // 32-sample words of a batch that any form takes
+
 // Binary-spike launches whose warps are all co-resident (32 to an SM) with
 // their edges in shared memory, and whose indexes fit 32 bits.
 static bool rs_fits(const BpArgs& a, int sm) {
-  if (a.res_cap <= 0 || a.smooth) return false;
+  if (a.res_cap <= 0 || a.smooth || a.KBs > kMaxWords) return false;
   const long long items = (long long)a.N * a.SL;
   if (items > (long long)sm * 32) return false;
   const long long warps = (items + sm - 1) / sm;
@@ -1070,7 +1072,7 @@ static int launch(bool forward, bool smooth, const BpArgs& a, int sm, cudaStream
   if (KB <= 1) return dispatch<1>(forward, smooth, a, sm, st);
   if (KB <= 2) return dispatch<2>(forward, smooth, a, sm, st);
   if (KB <= 4) return dispatch<4>(forward, smooth, a, sm, st);
-  if (KB <= 8) return dispatch<8>(forward, smooth, a, sm, st);
+  if (KB <= kMaxWords) return dispatch<8>(forward, smooth, a, sm, st);
   set_error("bptt: batch > 256");
   return SNC_B200_EUNSUPPORTED;
 }
