@@ -69,7 +69,6 @@ struct BpArgs {
   float* vsaved;       // K > 0: [T/K][N][B] v at segment ends; K == 0: [T][N][B] vp
   float* v;            // [N][B]
   const float* gspk;   // [T][N][B]
-  float* gw;           // [S]
   float* gext;         // [T][N][B] or null
   float* gv;           // [N][B]
   float* gcur;         // [R][N][B]
@@ -77,8 +76,9 @@ struct BpArgs {
   unsigned* ctl;
   int* err;
   int KBs;             // 32-sample words of a bit row: ceil(B / 32)
-  int SL, VB;          // batch slices of the weight gradient, words of a slice
-  float* part;         // [SL][S] weight gradient of every slice
+  int SL, VB, VB_log;  // batch slices of the weight gradient, words of a slice (1, 2 or 4)
+  int split;           // the sums are those of the resident launches
+  float* part;         // [SL][S] weight gradient of every slice (not split: the weight gradient)
   int Bp;              // samples of a padded row (SL * VB * 32)
   float* ring;         // resident backward: [R][N][Bp] future gradients
   int res_cap;         // resident launches: edges per direction staged per warp
@@ -288,14 +288,14 @@ __global__ void __launch_bounds__(kBpThreads, kBpMinBlocks<KB>) k_bptt_forward(B
 
 // One backward step for neuron i; vp_plane points at the [N][B] plane of
 // pre-reset potentials of step t.  sm_g: this warp's [B] scratch.
-template <int KB, bool SMOOTH, bool RES>
+template <int KB, bool SMOOTH, bool RES, bool SPLIT>
 __device__ __forceinline__ void bwd_neuron(const BpArgs& a, int t, int i, const float* vp_plane,
                                            float* sm_g, const WarpEdges& we) {
   const int lane = threadIdx.x & 31;
   const int N = a.N, B = a.B;
-  // two sums, each in edge order: the upstream gradient with the synapses of
-  // delay 2 and more, and those of delay 1 (k_res_backward takes the first
-  // before the barrier of the step)
+  // SPLIT: two sums, each in edge order: the upstream gradient with the synapses
+  // of delay 2 and more, and those of delay 1 (k_res_backward takes the first
+  // before the barrier of the step); else one
   float gs[KB], g1[KB];
   const size_t plane = ((size_t)t * N + i) * B;
 #pragma unroll
@@ -320,7 +320,7 @@ __device__ __forceinline__ void bwd_neuron(const BpArgs& a, int t, int i, const 
     // gradients (slot of t + d: one conditional subtraction, d < R) and a
     // validity bit; the batches below only broadcast them
     const unsigned okm = __ballot_sync(0xffffffffu, lane < n && t + my_d < a.T);
-    const unsigned onem = __ballot_sync(0xffffffffu, lane < n && my_d == 1);
+    const unsigned onem = SPLIT ? __ballot_sync(0xffffffffu, lane < n && my_d == 1) : 0u;
     size_t my_off = 0;
     if ((okm >> lane) & 1u) {
       const int slot = tr + my_d >= a.R ? tr + my_d - a.R : tr + my_d;
@@ -353,7 +353,7 @@ __device__ __forceinline__ void bwd_neuron(const BpArgs& a, int t, int i, const 
           for (int k = 0; k < KB; ++k) {
             const int b = 32 * k + lane;
             if (b >= B) continue;
-            if ((onem >> ((q0 + u) & 31)) & 1u) g1[k] = __fmaf_rn(wwv[u], gv[u][k], g1[k]);
+            if (SPLIT && (onem >> ((q0 + u) & 31)) & 1u) g1[k] = __fmaf_rn(wwv[u], gv[u][k], g1[k]);
             else gs[k] = __fmaf_rn(wwv[u], gv[u][k], gs[k]);
           }
     }
@@ -369,7 +369,7 @@ __device__ __forceinline__ void bwd_neuron(const BpArgs& a, int t, int i, const 
     const float s = SMOOTH ? __fdiv_rn(x, den) : (x >= 0.f ? 1.f : 0.f);
     const float sg = __fdiv_rn(1.f, __fmul_rn(den, den));
     const float gvv = a.gv[(size_t)i * B + b];
-    const float gst = __fsub_rn(__fadd_rn(gs[k], g1[k]), __fmul_rn(gvv, vp));
+    const float gst = __fsub_rn(SPLIT ? __fadd_rn(gs[k], g1[k]) : gs[k], __fmul_rn(gvv, vp));
     const float g = __fadd_rn(__fmul_rn(gvv, __fsub_rn(1.f, s)), __fmul_rn(gst, sg));
     gc[b] = g;
     if (a.gext) a.gext[plane + b] = g;
@@ -403,45 +403,46 @@ __device__ __forceinline__ void bwd_neuron(const BpArgs& a, int t, int i, const 
     for (int u = 0; u < 2; ++u) {
       if (ts[u] < 0) continue;
       const int eu = e + 32 * u;
-      // a sum per batch slice (one slice: the staged accumulator)
-      for (int sl = 0; sl < a.SL; ++sl) {
-        float c = 0.f;
-        if (!SMOOTH) {
-#pragma unroll
-          for (int k = 0; k < KB; ++k) {
-            if (k / a.VB != sl) continue;
-            uint32_t word = wv[u][k];
-            while (word) {
-              const int bb = __ffs(word) - 1;
-              c = __fadd_rn(c, sm_g[32 * k + bb]);
-              word &= word - 1u;
-            }
-          }
+      float c = 0.f;
+      auto add = [&](size_t slice) {  // to the weight gradient of one batch slice
+        if (c == 0.f) return;
+        if (RES) {
+          we.in_acc[eu] = __fadd_rn(we.in_acc[eu], c);
         } else {
-          const float* sp = a.spikes + ((size_t)ts[u] * N + pre[u]) * B;
-          for (int b = 32 * a.VB * sl; b < min(B, 32 * a.VB * (sl + 1)); ++b)
-            c = __fadd_rn(c, __fmul_rn(sm_g[b], sp[b]));
+          float* gp = a.part + slice * a.S + a.in_eidx[eu];
+          *gp = __fadd_rn(*gp, c);
         }
-        if (c != 0.f) {
-          if (RES && a.SL == 1) {
-            we.in_acc[eu] = __fadd_rn(we.in_acc[eu], c);
-          } else {
-            float* gp = a.part + (size_t)sl * a.S + (RES ? we.in_eidx[eu] : a.in_eidx[eu]);
-            *gp = __fadd_rn(*gp, c);
+      };
+      if (!SMOOTH) {
+#pragma unroll
+        for (int k = 0; k < KB; ++k) {
+          uint32_t word = wv[u][k];
+          while (word) {
+            const int bb = __ffs(word) - 1;
+            c = __fadd_rn(c, sm_g[32 * k + bb]);
+            word &= word - 1u;
+          }
+          // SPLIT: a sum per slice of VB words (KB is a multiple of VB)
+          if (SPLIT && ((k + 1) & (a.VB - 1)) == 0) {
+            add((size_t)(k >> a.VB_log));
+            c = 0.f;
           }
         }
+      } else {
+        const float* sp = a.spikes + ((size_t)ts[u] * N + pre[u]) * B;
+        for (int b = 0; b < B; ++b) c = __fadd_rn(c, __fmul_rn(sm_g[b], sp[b]));
       }
+      if (!SPLIT) add(0);
     }
   }
   __syncwarp();
 }
 
-// Resident launches of one slice: the warp's weight gradients, accumulated in
-// shared memory in the order the global form adds them, go out once.
+// Staged edges: the warp's weight gradients, accumulated in shared memory in the
+// order the global form adds them, go out once.
 __device__ __forceinline__ void flush_acc(const BpArgs& a, const WarpEdges& we) {
   const int lane = threadIdx.x & 31;
-  if (a.SL == 1)
-    for (int e = lane; e < we.nin; e += 32) a.part[we.in_eidx[e]] = we.in_acc[e];
+  for (int e = lane; e < we.nin; e += 32) a.part[we.in_eidx[e]] = we.in_acc[e];
 }
 
 // The weight gradient: the slices' sums in slice order.
@@ -453,7 +454,7 @@ __global__ void k_sum_slices(int S, int SL, const float* __restrict__ part, floa
   }
 }
 
-template <int KB, bool SMOOTH, bool RES>
+template <int KB, bool SMOOTH, bool RES, bool SPLIT>
 __global__ void __launch_bounds__(kBpThreads, kBpMinBlocks<KB>) k_bptt_backward(BpArgs a) {
   extern __shared__ float sm_all[];
   const int lane = threadIdx.x & 31;
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(kBpThreads, kBpMinBlocks<KB>) k_bptt_backward(
   if (a.K == 0) {
     for (int t = a.T - 1; t >= 0; --t) {
       for (int i = gw; i < a.N; i += W)
-        bwd_neuron<KB, SMOOTH, RES>(a, t, i, a.vsaved + (size_t)t * NB, sm_g, we);
+        bwd_neuron<KB, SMOOTH, RES, SPLIT>(a, t, i, a.vsaved + (size_t)t * NB, sm_g, we);
       target += nb;
       if (!grid_sync(&a.ctl[0], target, a.err, a.wait_ns)) return;
     }
@@ -508,7 +509,7 @@ __global__ void __launch_bounds__(kBpThreads, kBpMinBlocks<KB>) k_bptt_backward(
     }
     for (int t = t1 - 1; t >= t0; --t) {
       for (int i = gw; i < a.N; i += W)
-        bwd_neuron<KB, SMOOTH, RES>(a, t, i, a.seg + (size_t)(t - t0) * NB, sm_g, we);
+        bwd_neuron<KB, SMOOTH, RES, SPLIT>(a, t, i, a.seg + (size_t)(t - t0) * NB, sm_g, we);
       target += nb;
       if (!grid_sync(&a.ctl[0], target, a.err, a.wait_ns)) return;
     }
@@ -992,34 +993,61 @@ static int coop_launch(BpKernel kern, const BpArgs& a, int sm_count, size_t smem
   return SNC_B200_OK;
 }
 
-// A resident launch (a.res_cap > 0) when one warp per neuron can be
-// co-resident with the staged edges, else the global-memory form.
+// A launch with staged edges (smooth spikes, a.res_cap > 0) when one warp per
+// neuron can be co-resident with them, else the global-memory form.
 template <int KB>
 static int dispatch(bool forward, bool smooth, BpArgs a, int sm, cudaStream_t st) {
   const size_t smem = forward ? 0 : (size_t)(kBpThreads / 32) * 32 * KB * sizeof(float);
   if (smooth && a.res_cap > 0) {
     const size_t smem_r = smem + (size_t)(kBpThreads / 32) * 8 * a.res_cap * sizeof(int);
-    BpKernel kr = forward ? k_bptt_forward<KB, true, true> : k_bptt_backward<KB, true, true>;
+    BpKernel kr = forward ? k_bptt_forward<KB, true, true> : k_bptt_backward<KB, true, true, false>;
     if (resident_warps(kr, smem_r, sm) >= a.N) return coop_launch(kr, a, sm, smem_r, st);
   }
   a.res_cap = 0;
   BpKernel k = forward ? (smooth ? k_bptt_forward<KB, true, false> : k_bptt_forward<KB, false, false>)
-                       : (smooth ? k_bptt_backward<KB, true, false> : k_bptt_backward<KB, false, false>);
+                       : (smooth ? k_bptt_backward<KB, true, false, false>
+                          : a.split ? k_bptt_backward<KB, false, false, true>
+                                    : k_bptt_backward<KB, false, false, false>);
   return coop_launch(k, a, sm, smem, st);
 }
 
-// Batch slices of the weight gradient and of the resident launches: as many
-// warps as fit 32 to an SM, of 1, 2 or 4 words each (more warps hide more
-// latency: core of 1808 neurons, 128 samples, 1 slice of 4 words to 2 of 2).
-// Depends on the sizes alone, so that every form of a launch sums alike.
-static void pick_slices(BpArgs& a, int sm) {
+constexpr int kMaxWords = 8;  // 32-sample words of a batch that any form takes
+
+// Batch slices.  a.split: the resident launches can take this net and batch --
+// binary spikes, all warps co-resident (32 to an SM) with their edges in shared
+// memory (cap per direction; 0: too many), indexes of 32 bits -- in slices of
+// the fewest words (more warps hide more latency: core of 1808 neurons, 128
+// samples, 1 slice of 4 words to 2 of 2).  The global-memory form then sums in
+// their order, whether or not they are on.  Everything else is one slice, summed
+// in edge order: a sum per slice and two per gather cost the general form of 512
+// neurons of degree 300 at 128 samples 3.4 against 2.3 ms.
+static void pick_slices(BpArgs& a, int cap, int sm) {
   a.KBs = (a.B + 31) / 32;
-  int vb = 1;
-  while (vb < 4 && (long long)a.N * ((a.KBs + vb - 1) / vb) > (long long)sm * 32) vb <<= 1;
-  a.VB = vb;
-  a.SL = (a.KBs + vb - 1) / vb;
-  a.Bp = a.SL * vb * 32;
+  a.SL = 1;
+  a.split = 0;
+  if (a.smooth || cap <= 0 || a.KBs > kMaxWords) return;
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (((long long)a.T + a.R) * a.N * a.KBs >= INT_MAX || (long long)a.R * a.N >= INT_MAX / 2) return;
+  for (int lg = 0; lg <= 2; ++lg) {
+    const int vb = 1 << lg, sl = (a.KBs + vb - 1) / vb;
+    const long long items = (long long)a.N * sl, warps = (items + sm - 1) / sm;
+    const size_t ints = lg == 0 ? rs_warp_ints<1>(cap, true) : lg == 1 ? rs_warp_ints<2>(cap, true) : rs_warp_ints<4>(cap, true);
+    if (warps > 32 || ints * 4 * warps + 1024 > (size_t)optin ||
+        (long long)a.R * a.N * sl * vb * 128 > (long long)UINT_MAX)
+      continue;
+    a.split = 1;
+    a.VB = vb;
+    a.VB_log = lg;
+    a.SL = sl;
+    a.Bp = sl * vb * 32;
+    return;
+  }
 }
+
+// This launch is a resident one.
+static bool rs_takes(const BpArgs& a) { return a.split && a.res_cap > 0; }
 
 template <int VB>
 static int rs_launch(bool forward, const BpArgs& a, int sm, cudaStream_t st) {
@@ -1045,27 +1073,8 @@ static int rs_launch(bool forward, const BpArgs& a, int sm, cudaStream_t st) {
   return SNC_B200_OK;
 }
 
-constexpr int kMaxWords = 8;  // 32-sample words of a batch that any form takes
-
-// Binary-spike launches whose warps are all co-resident (32 to an SM) with
-// their edges in shared memory, and whose indexes fit 32 bits.
-static bool rs_fits(const BpArgs& a, int sm) {
-  if (a.res_cap <= 0 || a.smooth || a.KBs > kMaxWords) return false;
-  const long long items = (long long)a.N * a.SL;
-  if (items > (long long)sm * 32) return false;
-  const long long warps = (items + sm - 1) / sm;
-  int dev = 0, optin = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const size_t ints = a.VB == 1 ? rs_warp_ints<1>(a.res_cap, true)
-                      : a.VB == 2 ? rs_warp_ints<2>(a.res_cap, true) : rs_warp_ints<4>(a.res_cap, true);
-  return ints * 4 * warps + 1024 <= (size_t)optin &&
-         ((long long)a.T + a.R) * a.N * a.KBs < INT_MAX && (long long)a.R * a.N < INT_MAX / 2 &&
-         (long long)a.R * a.N * a.Bp * 4 <= (long long)UINT_MAX;
-}
-
 static int launch(bool forward, bool smooth, const BpArgs& a, int sm, cudaStream_t st) {
-  if (rs_fits(a, sm))
+  if (rs_takes(a))
     return a.VB == 1 ? rs_launch<1>(forward, a, sm, st)
            : a.VB == 2 ? rs_launch<2>(forward, a, sm, st) : rs_launch<4>(forward, a, sm, st);
   const int KB = a.KBs;
@@ -1088,9 +1097,9 @@ static int grow(T** p, size_t* cap, size_t n) {
   return rc;
 }
 
-// Edges per direction a resident launch stages per warp (0: none).
+// Edges per direction a resident launch stages per warp (0: too many).
 static int res_cap(const snc_b200_bptt* h) {
-  if (!h->resident || h->max_deg > kResCapMax) return 0;
+  if (h->max_deg > kResCapMax) return 0;
   return std::max(32, (h->max_deg + 31) / 32 * 32);
 }
 
@@ -1104,9 +1113,9 @@ static BpArgs forward_args(const snc_b200_bptt* h, const float* w, const float* 
   a.row_ptr = h->row_ptr; a.out_post = h->out_post; a.out_d = h->out_d; a.col_ptr = h->col_ptr;
   a.in_pre = h->in_pre; a.in_d = h->in_d; a.in_eidx = h->in_eidx;
   a.w = w; a.ext = ext; a.spikes = spikes; a.bits = spike_bits; a.vsaved = v_saved;
-  a.res_cap = res_cap(h);
+  a.res_cap = h->resident ? res_cap(h) : 0;
   a.even = h->even;
-  pick_slices(a, h->sm_count);
+  pick_slices(a, res_cap(h), h->sm_count);
   const WaitCtl wc = take_wait_ctl(true);
   a.wait_ns = wc.ns;
   a.stall = wc.stall;
@@ -1353,28 +1362,29 @@ int snc_b200_bptt_backward(snc_b200_bptt* h, const float* w, const float* ext, i
   a.in_pre = h->in_pre; a.in_d = h->in_d; a.in_eidx = h->in_eidx;
   a.w = w; a.ext = ext; a.spikes = const_cast<float*>(spikes);
   a.bits = const_cast<uint32_t*>(spike_bits); a.vsaved = const_cast<float*>(v_saved);
-  a.gspk = grad_spikes; a.gw = grad_w; a.gext = grad_ext;
+  a.gspk = grad_spikes; a.gext = grad_ext;
   a.ctl = h->ctl; a.err = h->err;
-  a.res_cap = res_cap(h);
+  a.res_cap = h->resident ? res_cap(h) : 0;
   a.even = h->even;
-  pick_slices(a, h->sm_count);
-  const bool rs = rs_fits(a, h->sm_count);
+  pick_slices(a, res_cap(h), h->sm_count);
+  const bool rs = rs_takes(a);
   // the resident form keeps its state in registers and pads its rows
   const size_t rows = rs ? (size_t)h->N * a.Bp : NB;
   if (!rs && (rc = grow(&h->v, &h->v_cap, NB))) return rc;
   if (!rs && (rc = grow(&h->gv, &h->gv_cap, NB))) return rc;
   if ((rc = grow(&h->gcur, &h->gcur_cap, (size_t)h->R * rows))) return rc;
   if (ckpt_every > 0 && (rc = grow(&h->seg, &h->seg_cap, (size_t)ckpt_every * rows))) return rc;
-  if ((rc = grow(&h->part, &h->part_cap, (size_t)a.SL * std::max(1, h->S)))) return rc;
-  a.v = h->v; a.gv = h->gv; a.gcur = h->gcur; a.ring = h->gcur; a.seg = h->seg; a.part = h->part;
+  if (a.split && (rc = grow(&h->part, &h->part_cap, (size_t)a.SL * std::max(1, h->S)))) return rc;
+  a.v = h->v; a.gv = h->gv; a.gcur = h->gcur; a.ring = h->gcur; a.seg = h->seg;
+  a.part = a.split ? h->part : grad_w;
   const WaitCtl wc = take_wait_ctl(true);
   a.wait_ns = wc.ns;
   a.stall = wc.stall;
   SNCB_CUDA(cudaMemsetAsync(h->ctl, 0, 16, st));
   SNCB_CUDA(cudaMemsetAsync(h->err, 0, 4, st));
-  if (!rs) SNCB_CUDA(cudaMemsetAsync(a.part, 0, (size_t)a.SL * std::max(1, h->S) * sizeof(float), st));
+  if (!rs) SNCB_CUDA(cudaMemsetAsync(a.part, 0, (size_t)a.SL * h->S * sizeof(float), st));
   if ((rc = launch(false, smooth != 0, a, h->sm_count, st))) return rc;
-  if (h->S > 0) {
+  if (a.split && h->S > 0) {
     k_sum_slices<<<std::min((h->S + 255) / 256, h->sm_count * 8), 256, 0, st>>>(h->S, a.SL, a.part, grad_w);
     SNCB_CUDA(cudaGetLastError());
   }
