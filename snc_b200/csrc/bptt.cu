@@ -79,7 +79,7 @@ struct BpArgs {
   int SL, VB, VB_log;  // batch slices of the weight gradient, words of a slice (1, 2 or 4)
   int split;           // the sums are those of the resident launches
   float* part;         // [SL][S] weight gradient of every slice (not split: the weight gradient)
-  int Bp;              // samples of a padded row (SL * VB * 32)
+  int Bp;              // resident backward: floats of a row (B, rounded up to VB)
   float* ring;         // resident backward: [R][N][Bp] future gradients
   int res_cap;         // resident launches: edges per direction staged per warp
   int even;            // resident launches: items in order, not round the CTAs
@@ -532,8 +532,9 @@ __global__ void __launch_bounds__(kBpThreads, kBpMinBlocks<KB>) k_bptt_backward(
 // synapses of delay 1.  Everything else -- the gather over the other synapses,
 // the weight gradient, the recomputation of a checkpoint segment -- runs
 // between the arrival at a step's barrier and the wait for it.  G lies in a
-// ring of padded rows, read as VB-wide vectors; rows of steps beyond T are
-// zero.  Edge offsets of a step are computed once per edge and passed through
+// ring whose rows start on VB floats, read as VB-wide vectors; lanes beyond the
+// batch read the next row (there is room behind the last) and drop what they
+// get.  Rows of steps beyond T are zero.  Edge offsets of a step are computed once per edge and passed through
 // shared memory.  The last steps, as many as the largest delay, stage the edges
 // anew with weight 0 for those that reach beyond T (an infinite weight times a
 // zero gradient would be NaN), so the gather needs no check; a check per offset
@@ -835,7 +836,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_backward(BpArgs a) {
     const int t0 = sg * K, t1 = min(T, t0 + K);
     const uint32_t* row = a.bits + (size_t)t0 * row_w;
     const float* ext = a.ext + ((size_t)t0 * N + j) * B + bf;
-    float* seg = a.seg + (size_t)j * a.Bp + bf;
+    float* seg = a.seg + (size_t)j * a.Bp + bf;  // rows as the ring's
     float v[VB];
 #pragma unroll
     for (int k = 0; k < VB; ++k)
@@ -855,7 +856,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_backward(BpArgs a) {
         const float vp = __fadd_rn(__fadd_rn(__fmul_rn(a.decay, v[k]), acc[k]), x_ext[k]);
         const float s = __fsub_rn(vp, a.thr) >= 0.f ? 1.f : 0.f;
         v[k] = __fmul_rn(vp, __fsub_rn(1.f, s));
-        seg[32 * k] = vp;
+        if (bf + 32 * k < B) seg[32 * k] = vp;
       }
       row += row_w;
       ext += (size_t)N * B;
@@ -903,7 +904,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_backward(BpArgs a) {
         if (bb + k >= B) g[k] = gv[k] = 0.f;
         reinterpret_cast<float*>(&out)[k] = g[k];
       }
-      *reinterpret_cast<Vec*>(a.ring + (size_t)(base + j) * a.Bp + bb) = out;
+      if (bb < B) *reinterpret_cast<Vec*>(a.ring + (size_t)(base + j) * a.Bp + bb) = out;
     }
     target += gridDim.x;
     grid_arrive(&a.ctl[0]);
@@ -1032,13 +1033,13 @@ static void pick_slices(BpArgs& a, int cap, int sm) {
     const long long items = (long long)a.N * sl, warps = (items + sm - 1) / sm;
     const size_t ints = lg == 0 ? rs_warp_ints<1>(cap, true) : lg == 1 ? rs_warp_ints<2>(cap, true) : rs_warp_ints<4>(cap, true);
     if (warps > 32 || ints * 4 * warps + 1024 > (size_t)optin ||
-        (long long)a.R * a.N * sl * vb * 128 > (long long)UINT_MAX)
+        ((long long)a.R * a.N + 1) * sl * vb * 128 > (long long)UINT_MAX)
       continue;
     a.split = 1;
     a.VB = vb;
     a.VB_log = lg;
     a.SL = sl;
-    a.Bp = sl * vb * 32;
+    a.Bp = (a.B + vb - 1) / vb * vb;
     return;
   }
 }
@@ -1365,12 +1366,13 @@ int snc_b200_bptt_backward(snc_b200_bptt* h, const float* w, const float* ext, i
   a.even = h->even;
   pick_slices(a, res_cap(h), h->sm_count);
   const bool rs = rs_takes(a);
-  // the resident form keeps its state in registers and pads its rows
-  const size_t rows = rs ? (size_t)h->N * a.Bp : NB;
+  // the resident form keeps its state in registers; its lanes beyond the batch
+  // read behind the last rows
+  const size_t rows = rs ? (size_t)h->N * a.Bp : NB, behind = rs ? (size_t)a.SL * a.VB * 32 : 0;
   if (!rs && (rc = grow(&h->v, &h->v_cap, NB))) return rc;
   if (!rs && (rc = grow(&h->gv, &h->gv_cap, NB))) return rc;
-  if ((rc = grow(&h->gcur, &h->gcur_cap, (size_t)h->R * rows))) return rc;
-  if (ckpt_every > 0 && (rc = grow(&h->seg, &h->seg_cap, (size_t)ckpt_every * rows))) return rc;
+  if ((rc = grow(&h->gcur, &h->gcur_cap, (size_t)h->R * rows + behind))) return rc;
+  if (ckpt_every > 0 && (rc = grow(&h->seg, &h->seg_cap, (size_t)ckpt_every * rows + behind))) return rc;
   if (a.split && (rc = grow(&h->part, &h->part_cap, (size_t)a.SL * std::max(1, h->S)))) return rc;
   a.v = h->v; a.gv = h->gv; a.gcur = h->gcur; a.ring = h->gcur; a.seg = h->seg;
   a.part = a.split ? h->part : grad_w;
