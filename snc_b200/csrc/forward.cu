@@ -407,11 +407,11 @@ __device__ void apply_ordered(const G& grp, int ce, int* head, int* tail, int nc
 }
 
 constexpr int kSThreads = 1024;
-enum { kSAtomic = 0, kSOrdered = 1, kSLean = 2 };  // deliveries of the tier-S kernel
+enum { kSAtomic = 0, kSOrdered = 1 };  // deliveries of the tier-S kernel
 constexpr int kSRows = 4;   // fired rows of a lane: a tier-S warp takes 128 at once
 constexpr int kSAhead = 2;  // 32-event groups whose edges a tier-S warp keeps in flight
-constexpr int kSTags = 512; // bytes of a warp's own tags where every cell cannot have one
-constexpr int kSScratch = 32 * kSRows + 32 + 4;  // ints of scratch of a tier-S warp
+// ints of scratch of a tier-S warp that stages up to cap rows
+__host__ __device__ constexpr int s_scratch(int cap) { return (cap < 32 * kSRows ? cap : 32 * kSRows) + 32 + 4; }
 constexpr int kSOff = kSPtr + 1;  // ints of a staged row (odd: no bank conflicts)
 
 // Barrier of the thread-block cluster; orders shared-memory writes of its CTAs
@@ -443,15 +443,6 @@ __device__ __forceinline__ void sts_i(unsigned a, int v) {
 __device__ __forceinline__ void sts_f(unsigned a, float v) { sts_i(a, __float_as_int(v)); }
 __device__ __forceinline__ void sts_b(unsigned a, int v) {
   asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-
-// Adds the events of one 32-event group whose cells (shared addresses) may
-// coincide: rank is an event's place among the group's events of its cell.
-__device__ __forceinline__ void add_ranked(bool valid, unsigned cell, float w, int rank) {
-  for (int r = 0; __any_sync(0xffffffffu, valid && rank >= r); ++r) {
-    if (valid && rank == r) sts_f(cell, __fadd_rn(lds_f(cell), w));
-    __syncwarp();
-  }
 }
 
 // Copies the segment starts of row j (and the end of its last segment) to
@@ -524,19 +515,19 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
   int* off = reinterpret_cast<int*>(psi + (inl ? nc : 0));  // [s_cap][kSOff] staged rows
   // per warp: segment offsets and segment marks
   int* scr0 = off + (DEL != kSOrdered ? 0 : a.s_cap * kSOff);
-  int* scr = scr0 + (DEL != kSOrdered ? 0 : warp * kSScratch);
-  unsigned* mark = reinterpret_cast<unsigned*>(scr + 32 * kSRows);
-  unsigned short* fired = reinterpret_cast<unsigned short*>(scr0 + (DEL != kSOrdered ? 0 : nwarps * kSScratch));
-  // a byte per cell, or kSTags per warp
-  unsigned char* tag = reinterpret_cast<unsigned char*>(fired + N) + (a.s_tmask == kSTags - 1 ? warp * kSTags : 0);
+  const int n_scr = s_scratch(a.s_cap);
+  unsigned* mark = reinterpret_cast<unsigned*>(scr0 + (DEL != kSOrdered ? 0 : warp * n_scr));
+  unsigned short* fired = reinterpret_cast<unsigned short*>(scr0 + (DEL != kSOrdered ? 0 : nwarps * n_scr));
+  // a byte per cell, or s_tmask + 1 per warp
+  unsigned char* tag = reinterpret_cast<unsigned char*>(fired + N) + (a.s_tmask == INT_MAX ? 0 : warp * (a.s_tmask + 1));
   const int tmask = a.s_tmask;
   const LifP lif = a.lif;
   const float thr = lif.thr;
   // the delivery's arrays as shared addresses
   const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring);
   const unsigned off_w = (unsigned)__cvta_generic_to_shared(off + lane * kSOff + warp);
-  const unsigned scr_s = (unsigned)__cvta_generic_to_shared(scr);
   const unsigned mark_s = (unsigned)__cvta_generic_to_shared(mark);
+  const unsigned scr_s = mark_s + 4 * 36;
   const unsigned tag_s = (unsigned)__cvta_generic_to_shared(tag);
   const unsigned upto = below | (1u << lane);
   const uint2* __restrict__ sed = a.sedges;
@@ -782,29 +773,6 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
             }
           }
         }
-      } else if (DEL == kSLean) {
-        // lane l: this warp's segment of fired row k0 + l, one after another
-        if (warp < kSRanges)
-          for (int k0 = 0; k0 < nf; k0 += 32) {
-            int st = 0, ln = 0;
-            if (k0 + lane < nf) {
-              const int* op = a.sptr + fired[k0 + lane] * kSPtr + warp;
-              st = op[0];
-              ln = op[1] - st;
-            }
-            for (unsigned ne = __ballot_sync(0xffffffffu, ln > 0); ne; ne &= ne - 1u) {
-              const int l = __ffs(ne) - 1;
-              const int s = __shfl_sync(0xffffffffu, st, l), n = __shfl_sync(0xffffffffu, ln, l);
-              n_events += n;
-              for (int e0 = 0; e0 < n; e0 += 32) {
-                const bool valid = e0 + lane < n;
-                const uint2 ed = valid ? a.sedges[s + e0 + lane] : make_uint2(0u, 0u);
-                const unsigned cell = cell_at(ed.x);
-                const unsigned peers = __match_any_sync(0xffffffffu, valid ? (int)cell : -1 - lane);
-                add_ranked(valid, cell, __uint_as_float(ed.y), __popc(peers & below));
-              }
-            }
-          }
       } else {
         for (int r0 = 0;;) {
           const int nb = min(a.s_cap, nf - r0);
@@ -1785,23 +1753,24 @@ static SPlan tier_s_layout(const Graph* g, const SLayout& L, int noc, bool inl, 
   p.smem = base(p.kn);
   if (mode != MODE_SORT && L.cl == 1) return p;
   p.del = kSOrdered;
-  const size_t b0 = p.smem + nw * kSScratch * 4;
   // a tag per cell before tags per warp (their false conflicts cost more than
-  // a second round of staging), then the larger stage
-  for (const bool exact : {true, false})
-    for (const int cap : {256, 128}) {
-      const size_t need = b0 + (size_t)cap * kSOff * 4 + (exact ? cells : nw * kSTags);
-      if (need <= budget) {
-        p.cap = cap;
-        p.tmask = exact ? INT_MAX : kSTags - 1;
-        p.smem = need;
-        return p;
-      }
-    }
-  p.kn = 0;
-  p.del = kSLean;
-  p.smem = base(0);
-  return p;
+  // a second round of staging), then the larger stage; states that leave little
+  // room stage few rows at once (one CTA: the last of these always fits beside a
+  // state that tier_s_bytes admits).  380 neurons, delays to 149, 240 events a
+  // step: 2.2 us a step, 7.3 with a warp's segments one row after another and no
+  // scratch, 3.2 with events staged 1024 at a time
+  const size_t state = p.smem;
+  const struct { int cap, tags; } plans[] = {{256, 0},  {128, 0},  {256, 512}, {128, 512},
+                                             {64, 512}, {64, 256}, {32, 256},  {32, 128}};
+  for (const auto& c : plans) {
+    if (L.cl > 1 && c.cap < 128) break;
+    p.smem = state + nw * s_scratch(c.cap) * 4 + (size_t)c.cap * kSOff * 4 + (c.tags ? nw * c.tags : cells);
+    if (p.smem > budget) continue;
+    p.cap = c.cap;
+    p.tmask = c.tags ? c.tags - 1 : INT_MAX;
+    return p;
+  }
+  return p;  // cap 0: none
 }
 
 // A launch of cl CTAs for each of `samples` samples; attr: one attribute, kept
@@ -1827,7 +1796,6 @@ static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, cons
   using Kern = void (*)(FwdArgs);
   auto pick = [&](int kn, int del) -> Kern {
     if (L.cl > 1) return k_tier_s<1, EP, kSOrdered, kSCluster>;
-    if (del == kSLean) return k_tier_s<0, EP, kSLean, 1>;
     if (del == kSAtomic)
       return kn == 1 ? k_tier_s<1, EP, kSAtomic, 1> : kn == 2 ? k_tier_s<2, EP, kSAtomic, 1>
              : kn == 4 ? k_tier_s<4, EP, kSAtomic, 1> : k_tier_s<0, EP, kSAtomic, 1>;
@@ -1843,8 +1811,8 @@ static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, cons
   SNCB_CUDA(cudaFuncGetAttributes(&fa, pick(2, kSOrdered)));
   const size_t budget = (size_t)optin_smem() - fa.sharedSizeBytes;
   const SPlan p = tier_s_layout(g, L, a.noc, EP && a.elig, mode, budget);
-  if (L.cl > 1 && p.del != kSOrdered) {  // (no such layout is built: tier_s_clusters)
-    set_error("tier S: a cluster's part does not fit on an SM");
+  if (p.del == kSOrdered && !p.cap) {  // (no such cluster layout is built: tier_s_clusters)
+    set_error("tier S: a sample's state does not fit on an SM");
     return SNC_B200_EUNSUPPORTED;
   }
   a.s_cap = p.cap;
@@ -2059,7 +2027,7 @@ int tier_s_clusters(const Graph* g, const SLayout& L) {
     bool ok = cudaFuncGetAttributes(&fa, kern) == cudaSuccess;
     const size_t budget = (size_t)optin_smem() - std::min((size_t)optin_smem(), fa.sharedSizeBytes);
     const SPlan p = tier_s_layout(g, L, std::max(1, g->noc), false, MODE_SORT, budget);
-    ok = ok && p.del == kSOrdered &&
+    ok = ok && p.cap > 0 &&
          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) == cudaSuccess;
     if (ok) {
       cudaLaunchAttribute attr[1];
