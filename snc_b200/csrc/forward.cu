@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
   int* off = reinterpret_cast<int*>(psi + (inl ? nc : 0));  // [s_cap][kSOff] staged rows
   // per warp: segment offsets and segment marks
   int* scr0 = off + (DEL != kSOrdered ? 0 : a.s_cap * kSOff);
-  const int n_scr = s_scratch(a.s_cap);
+  const int n_scr = s_scratch(CL > 1 ? 32 * kSRows : a.s_cap);  // (clusters: 128 rows and more)
   unsigned* mark = reinterpret_cast<unsigned*>(scr0 + (DEL != kSOrdered ? 0 : warp * n_scr));
   unsigned short* fired = reinterpret_cast<unsigned short*>(scr0 + (DEL != kSOrdered ? 0 : nwarps * n_scr));
   // a byte per cell, or s_tmask + 1 per warp
@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
 #pragma unroll
             for (int i = 0; i < kSRows; ++i) {
               st[i] = ln[i] = pos[i] = 0;
-              if (i >= nr) continue;  // warp-uniform
+              if (KN && i >= nr) continue;  // warp-uniform; large nets fill them
               if (k0 + 32 * i + lane < nb) {
                 const unsigned op = off_w + 4u * ((k0 + 32 * i) * kSOff);
                 st[i] = lds_i(op);
@@ -1734,7 +1734,8 @@ static int optin_smem() {
 }
 
 // Launch shape of the tier-S kernel: neurons of a thread held in registers
-// (1, 2 or 4; 0: state in shared memory), the delivery, fired rows staged at
+// (1 or 2; 0: state in shared memory, beyond 2048 neurons -- four in registers
+// took 13.5 us a step for 3000 neurons, 11.5 so), the delivery, fired rows staged at
 // once, mask of the conflict tags, bytes of dynamic shared memory.
 struct SPlan {
   int kn, del, cap, tmask;
@@ -1744,7 +1745,7 @@ struct SPlan {
 static SPlan tier_s_layout(const Graph* g, const SLayout& L, int noc, bool inl, int mode, size_t budget) {
   const int nch = std::max(1, (g->N + kSThreads * L.cl - 1) / (kSThreads * L.cl));
   const size_t cells = (size_t)g->R * L.ncols, nw = kSThreads / 32;
-  SPlan p{nch <= 1 ? 1 : nch <= 2 ? 2 : nch <= 4 ? 4 : 0, kSAtomic, 0, 0, 0};
+  SPlan p{nch <= 1 ? 1 : nch <= 2 ? 2 : 0, kSAtomic, 0, 0, 0};
   auto base = [&](int kn) {
     const size_t cnt = L.cl > 1 ? 2 * ((size_t)g->N + 31) / 32 + 2 : (size_t)(kn ? kn : nch) * nw;
     return (cells + g->N + noc + cnt + (kn ? 0 : 2 * (size_t)g->N) +
@@ -1760,8 +1761,8 @@ static SPlan tier_s_layout(const Graph* g, const SLayout& L, int noc, bool inl, 
   // step: 2.2 us a step, 7.3 with a warp's segments one row after another and no
   // scratch, 3.2 with events staged 1024 at a time
   const size_t state = p.smem;
-  const struct { int cap, tags; } plans[] = {{256, 0},  {128, 0},  {256, 512}, {128, 512},
-                                             {64, 512}, {64, 256}, {32, 256},  {32, 128}};
+  const struct { int cap, tags; } plans[] = {{g->N > 2048 ? 512 : 256, 0}, {256, 0},  {128, 0},  {256, 512},
+                                             {128, 512}, {64, 512}, {64, 256}, {32, 256}, {32, 128}};
   for (const auto& c : plans) {
     if (L.cl > 1 && c.cap < 128) break;
     p.smem = state + nw * s_scratch(c.cap) * 4 + (size_t)c.cap * kSOff * 4 + (c.tags ? nw * c.tags : cells);
@@ -1798,9 +1799,9 @@ static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, cons
     if (L.cl > 1) return k_tier_s<1, EP, kSOrdered, kSCluster>;
     if (del == kSAtomic)
       return kn == 1 ? k_tier_s<1, EP, kSAtomic, 1> : kn == 2 ? k_tier_s<2, EP, kSAtomic, 1>
-             : kn == 4 ? k_tier_s<4, EP, kSAtomic, 1> : k_tier_s<0, EP, kSAtomic, 1>;
+                                                             : k_tier_s<0, EP, kSAtomic, 1>;
     return kn == 1 ? k_tier_s<1, EP, kSOrdered, 1> : kn == 2 ? k_tier_s<2, EP, kSOrdered, 1>
-           : kn == 4 ? k_tier_s<4, EP, kSOrdered, 1> : k_tier_s<0, EP, kSOrdered, 1>;
+                                                            : k_tier_s<0, EP, kSOrdered, 1>;
   };
   if (L.cl > 1 && EP && a.elig) {
     // its CTAs hold the surrogates of their own columns only
