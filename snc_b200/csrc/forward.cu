@@ -1388,8 +1388,6 @@ __device__ void phase_b(const G& grp, const FwdArgs& a, const GSmem& sm, int* sc
   // read the descriptor slots of the fast path in the same round trip as the
   // count (slots beyond the count hold stale descriptors and are ignored)
   const int cap = sm.ib[b + 1] - sm.ib[b];
-  // two descriptors a thread in the scan (a CTA has kGThreads at least)
-  const int dcap = G::kGroups > 1 ? min(kGDesc, 2 * nthr) : kGDesc;
   unsigned long long spec = 0, spec2 = 0;
   if (tid < 32 && tid < cap) spec = __ldcg(&box[tid]);
   if (MODE == MODE_SORT && tid < 32 && tid + 32 < cap) spec2 = __ldcg(&box[tid + 32]);
@@ -1407,15 +1405,15 @@ __device__ void phase_b(const G& grp, const FwdArgs& a, const GSmem& sm, int* sc
   if (cnt <= (MODE == MODE_SORT ? kFastDesc : 32) &&
       phase_b_fast<MODE, RSM>(grp, a, sm, k, s0, cb0, cnt, spec, spec2, tail_sync))
     return;
-  if (MODE == MODE_SORT && cnt > dcap) {
+  if (MODE == MODE_SORT && cnt > kGDesc) {
     phase_b_scan<RSM>(grp, a, sm, scratch, k, t, s0, b, cb0, cb1);
     return;
   }
   float* rb = ring_base<RSM>(a, sm, k);
   const int stride = RSM ? a.BS : a.ncols;
   const int col0 = RSM ? 0 : cb0;
-  for (int d0 = 0; d0 < cnt; d0 += dcap) {
-    const int dn = min(dcap, cnt - d0);
+  for (int d0 = 0; d0 < cnt; d0 += kGDesc) {
+    const int dn = min(kGDesc, cnt - d0);
     for (int i = tid; i < dn; i += nthr) sm.desc[i] = __ldcg(&box[d0 + i]);
     grp.sync();
     const unsigned long long* src = sm.desc;
@@ -1454,13 +1452,18 @@ __device__ void phase_b(const G& grp, const FwdArgs& a, const GSmem& sm, int* sc
         grp.sync();
         src = sm.dsort;
       }
-      // prefix of segment lengths, two descriptors per thread
-      const int i0 = 2 * tid, i1 = 2 * tid + 1;
-      const int l0 = i0 < dn ? (int)(src[i0] & 0xffffffffu) : 0;
-      const int l1 = i1 < dn ? (int)(src[i1] & 0xffffffffu) : 0;
-      const int ex = group_exclusive_scan(grp, l0 + l1, scratch, &E);
-      if (i0 < dn) sm.seg_p[i0] = ex;
-      if (i1 < dn) sm.seg_p[i1] = ex + l0;
+      // prefix of segment lengths, two descriptors per thread at a time
+      E = 0;
+      for (int q0 = 0; q0 < dn; q0 += 2 * nthr) {
+        const int i0 = q0 + 2 * tid, i1 = i0 + 1;
+        const int l0 = i0 < dn ? (int)(src[i0] & 0xffffffffu) : 0;
+        const int l1 = i1 < dn ? (int)(src[i1] & 0xffffffffu) : 0;
+        int part;
+        const int ex = E + group_exclusive_scan(grp, l0 + l1, scratch, &part);
+        if (i0 < dn) sm.seg_p[i0] = ex;
+        if (i1 < dn) sm.seg_p[i1] = ex + l0;
+        E += part;
+      }
       grp.sync();
     }
     for (int e0 = 0; e0 < E; e0 += kGChunk) {
