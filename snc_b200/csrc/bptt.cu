@@ -78,7 +78,7 @@ struct BpArgs {
   int KBs;             // 32-sample words of a bit row: ceil(B / 32)
   int SL, VB, VB_log;  // batch slices of the weight gradient, words of a slice (1, 2 or 4)
   int split;           // the sums are those of the resident launches
-  float* part;         // [SL][S] weight gradient of every slice (not split: the weight gradient)
+  float* part;         // [SL][S] weight gradient of every slice (one: the weight gradient)
   int Bp;              // resident backward: floats of a row (B, rounded up to VB)
   float* ring;         // resident backward: [R][N][Bp] future gradients
   int res_cap;         // resident launches: edges per direction staged per warp
@@ -1373,9 +1373,9 @@ int snc_b200_bptt_backward(snc_b200_bptt* h, const float* w, const float* ext, i
   if (!rs && (rc = grow(&h->gv, &h->gv_cap, NB))) return rc;
   if ((rc = grow(&h->gcur, &h->gcur_cap, (size_t)h->R * rows + behind))) return rc;
   if (ckpt_every > 0 && (rc = grow(&h->seg, &h->seg_cap, (size_t)ckpt_every * rows + behind))) return rc;
-  if (a.split && (rc = grow(&h->part, &h->part_cap, (size_t)a.SL * std::max(1, h->S)))) return rc;
+  if (a.SL > 1 && (rc = grow(&h->part, &h->part_cap, (size_t)a.SL * std::max(1, h->S)))) return rc;
   a.v = h->v; a.gv = h->gv; a.gcur = h->gcur; a.ring = h->gcur; a.seg = h->seg;
-  a.part = a.split ? h->part : grad_w;
+  a.part = a.SL > 1 ? h->part : grad_w;
   const WaitCtl wc = take_wait_ctl(true);
   a.wait_ns = wc.ns;
   a.stall = wc.stall;
@@ -1384,7 +1384,7 @@ int snc_b200_bptt_backward(snc_b200_bptt* h, const float* w, const float* ext, i
   if (rs) SNCB_CUDA(cudaMemsetAsync(a.ring, 0, (size_t)h->R * rows * sizeof(float), st));
   else SNCB_CUDA(cudaMemsetAsync(a.part, 0, (size_t)a.SL * h->S * sizeof(float), st));
   if ((rc = launch(false, smooth != 0, a, h->sm_count, st))) return rc;
-  if (a.split && h->S > 0) {
+  if (a.SL > 1 && h->S > 0) {
     k_sum_slices<<<std::min((h->S + 255) / 256, h->sm_count * 8), 256, 0, st>>>(h->S, a.SL, a.part, grad_w);
     SNCB_CUDA(cudaGetLastError());
   }
