@@ -1139,36 +1139,57 @@ using namespace sncb;
 // x[t] (reverse: from the last step backwards, y[t] = decay * y[t+1] + x[t]),
 // each product and sum rounded separately like the step-by-step loop of the
 // readouts (shd_model.py:139-140, lm.py:90); the reverse form is its
-// gradient.  A thread takes W neighbouring columns, eight steps' loads at once:
-// one 4-byte load a step in flight moved 268 MB in and out in 111 us, eight of
-// 16 bytes in 82, the rate of a plain copy (4096 x 64 columns, 256 steps).
+// gradient.  A thread takes W neighbouring columns, the loads of several steps at
+// once.  Four columns where there are many: 268 MB in and out (4096 x 64 columns,
+// 256 steps) in 83 us, the rate of a plain copy, 111 with a 4-byte load a step.
+// One column where there are few, and then a thread's own chain of steps is what
+// counts: it requests 16 steps while it adds the 16 before (64 columns, 1000
+// steps: 20 us, 69 with eight requested behind each other's sums).
 template <int W>
 __global__ void k_leaky_scan(const float* __restrict__ x, float* __restrict__ y, int T, long long n,
                              float decay, int reverse) {
-  constexpr int U = 8;
+  constexpr int U = W == 1 ? 16 : 8;
   struct alignas(4 * W) Vec {
     float v[W];
   };
+  const long long step = reverse ? -n : n, first = reverse ? (T - 1) * n : 0;
   for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n / W;
        j += (long long)gridDim.x * blockDim.x) {
+    const float* p = x + first + j * W;
+    float* q = y + first + j * W;
     float acc[W];
 #pragma unroll
     for (int i = 0; i < W; ++i) acc[i] = 0.f;
-    for (int k0 = 0; k0 < T; k0 += U) {
-      Vec in[U];
+    auto get = [&](Vec (&s)[U]) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const long long t = reverse ? T - 1 - k0 - u : k0 + u;
-        if (k0 + u < T) in[u] = *reinterpret_cast<const Vec*>(x + t * n + j * W);
-      }
+      for (int u = 0; u < U; ++u, p += step) s[u] = *reinterpret_cast<const Vec*>(p);
+    };
+    auto put = [&](Vec& s) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const long long t = reverse ? T - 1 - k0 - u : k0 + u;
-        if (k0 + u >= T) break;
+      for (int i = 0; i < W; ++i) s.v[i] = acc[i] = __fadd_rn(__fmul_rn(decay, acc[i]), s.v[i]);
+      *reinterpret_cast<Vec*>(q) = s;
+      q += step;
+    };
+    int left = T;
+    Vec in[U];
+    if (W == 1 && left >= U) get(in);
+    for (; left >= (W == 1 ? 2 * U : U); left -= U) {
+      Vec next[U];
+      get(W == 1 ? next : in);
 #pragma unroll
-        for (int i = 0; i < W; ++i) in[u].v[i] = acc[i] = __fadd_rn(__fmul_rn(decay, acc[i]), in[u].v[i]);
-        *reinterpret_cast<Vec*>(y + t * n + j * W) = in[u];
-      }
+      for (int u = 0; u < U; ++u) put(in[u]);
+      if (W == 1)
+#pragma unroll
+        for (int u = 0; u < U; ++u) in[u] = next[u];
+    }
+    if (W == 1 && left >= U) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) put(in[u]);
+      left -= U;
+    }
+    for (; left > 0; --left, p += step) {
+      Vec s = *reinterpret_cast<const Vec*>(p);
+      put(s);
     }
   }
 }
