@@ -407,7 +407,8 @@ __device__ void apply_ordered(const G& grp, int ce, int* head, int* tail, int nc
 }
 
 constexpr int kSThreads = 1024;
-enum { kSAtomic = 0, kSOrdered = 1 };  // deliveries of the tier-S kernel
+// deliveries of the tier-S kernel (kSRoom: ordered, fewer than 128 rows staged)
+enum { kSAtomic = 0, kSOrdered = 1, kSRoom = 2 };
 constexpr int kSRows = 4;   // fired rows of a lane: a tier-S warp takes 128 at once
 constexpr int kSAhead = 2;  // 32-event groups whose edges a tier-S warp keeps in flight
 // ints of scratch of a tier-S warp that stages up to cap rows
@@ -513,11 +514,15 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
   const bool inl = EP && a.elig;
   float* psi = tr + (inl ? N : 0);
   int* off = reinterpret_cast<int*>(psi + (inl ? nc : 0));  // [s_cap][kSOff] staged rows
-  // per warp: segment offsets and segment marks
-  int* scr0 = off + (DEL != kSOrdered ? 0 : a.s_cap * kSOff);
-  const int n_scr = s_scratch(CL > 1 ? 32 * kSRows : a.s_cap);  // (clusters: 128 rows and more)
-  unsigned* mark = reinterpret_cast<unsigned*>(scr0 + (DEL != kSOrdered ? 0 : warp * n_scr));
-  unsigned short* fired = reinterpret_cast<unsigned short*>(scr0 + (DEL != kSOrdered ? 0 : nwarps * n_scr));
+  // per warp: segment offsets and segment marks.
+  int* scr0 = off + (DEL == kSAtomic ? 0 : a.s_cap * kSOff);
+  // 128 rows' segments and then the marks, at constant places, where that measured
+  // faster (70 samples of a 998-neuron net 494 us, 504 in the other order); else
+  // the marks first and as many segments as are staged
+  constexpr bool kFull = DEL == kSOrdered && KN == 1 && (!EP || CL > 1);
+  const int n_scr = s_scratch(kFull ? 32 * kSRows : a.s_cap);
+  unsigned* mark = reinterpret_cast<unsigned*>(scr0 + (DEL == kSAtomic ? 0 : warp * n_scr) + (kFull ? 32 * kSRows : 0));
+  unsigned short* fired = reinterpret_cast<unsigned short*>(scr0 + (DEL == kSAtomic ? 0 : nwarps * n_scr));
   // a byte per cell, or s_tmask + 1 per warp
   unsigned char* tag = reinterpret_cast<unsigned char*>(fired + N) + (a.s_tmask == INT_MAX ? 0 : warp * (a.s_tmask + 1));
   const int tmask = a.s_tmask;
@@ -527,7 +532,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
   const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring);
   const unsigned off_w = (unsigned)__cvta_generic_to_shared(off + lane * kSOff + warp);
   const unsigned mark_s = (unsigned)__cvta_generic_to_shared(mark);
-  const unsigned scr_s = mark_s + 4 * 36;
+  const unsigned scr_s = kFull ? mark_s - 4 * 32 * kSRows : mark_s + 4 * 36;
   const unsigned tag_s = (unsigned)__cvta_generic_to_shared(tag);
   const unsigned upto = below | (1u << lane);
   const uint2* __restrict__ sed = a.sedges;
@@ -710,7 +715,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tier_s(FwdArgs a) {
           unsigned m = __ballot_sync(0xffffffffu, f);
           if (!m) continue;
           if (f) fired[rk + __popc(m & below)] = (unsigned short)(c * nthr + tid);
-          if (DEL == kSOrdered)
+          if (DEL != kSAtomic)
             for (; m && rk < a.s_cap; m &= m - 1u, ++rk)
               stage_row(a.sptr, c * nthr + warp * 32 + __ffs(m) - 1, off + rk * kSOff, lane);
         }
@@ -1798,11 +1803,12 @@ template <bool EP>
 static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, const FwdArgs& a_in, cudaStream_t st) {
   FwdArgs a = a_in;
   using Kern = void (*)(FwdArgs);
-  auto pick = [&](int kn, int del) -> Kern {
+  auto pick = [&](int kn, int del, int cap) -> Kern {
     if (L.cl > 1) return k_tier_s<1, EP, kSOrdered, kSCluster>;
     if (del == kSAtomic)
       return kn == 1 ? k_tier_s<1, EP, kSAtomic, 1> : kn == 2 ? k_tier_s<2, EP, kSAtomic, 1>
                                                              : k_tier_s<0, EP, kSAtomic, 1>;
+    if (!EP && kn == 1 && cap < 32 * kSRows) return k_tier_s<1, EP, kSRoom, 1>;
     return kn == 1 ? k_tier_s<1, EP, kSOrdered, 1> : kn == 2 ? k_tier_s<2, EP, kSOrdered, 1>
                                                             : k_tier_s<0, EP, kSOrdered, 1>;
   };
@@ -1812,7 +1818,7 @@ static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, cons
     return SNC_B200_EUNSUPPORTED;
   }
   cudaFuncAttributes fa{};
-  SNCB_CUDA(cudaFuncGetAttributes(&fa, pick(2, kSOrdered)));
+  SNCB_CUDA(cudaFuncGetAttributes(&fa, pick(2, kSOrdered, 0)));
   const size_t budget = (size_t)optin_smem() - fa.sharedSizeBytes;
   const SPlan p = tier_s_layout(g, L, a.noc, EP && a.elig, mode, budget);
   if (p.del == kSOrdered && !p.cap) {  // (no such cluster layout is built: tier_s_clusters)
@@ -1824,7 +1830,7 @@ static int launch_tier_s(const Graph* g, const SLayout& L, int B, int mode, cons
   a.s_nc = L.ncols;
   a.s_col = L.col;
   a.sptr = L.sptr;
-  const Kern kern = pick(p.kn, p.del);
+  const Kern kern = pick(p.kn, p.del, p.cap);
   SNCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
   int per_sm = 0;
   SNCB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSThreads, p.smem));
