@@ -79,7 +79,7 @@ struct BpArgs {
   int SL, VB, VB_log;  // batch slices of the weight gradient, words of a slice (1, 2 or 4)
   int split;           // the sums are those of the resident launches
   float* part;         // [SL][S] weight gradient of every slice (one: the weight gradient)
-  int Bp;              // resident backward: floats of a row (B, rounded up to VB)
+  int Bp;              // resident backward: floats of a row (B, rounded up to 8, a smaller batch to VB)
   float* ring;         // resident backward: [R][N][Bp] future gradients
   int res_cap;         // resident launches: edges per direction staged per warp
   int even;            // resident launches: items in order, not round the CTAs
@@ -1039,7 +1039,8 @@ static void pick_slices(BpArgs& a, int cap, int sm) {
     a.VB = vb;
     a.VB_log = lg;
     a.SL = sl;
-    a.Bp = (a.B + vb - 1) / vb * vb;
+    const int unit = a.B < 8 ? vb : 8;  // whole 32-byte sectors, where rows have any
+    a.Bp = (a.B + unit - 1) / unit * unit;
     return;
   }
 }
