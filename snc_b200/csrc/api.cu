@@ -100,6 +100,7 @@ static int validate_view(const snc_graph_view* v) {
 }
 
 void free_graph(Graph* g) {
+  const PoolBatch batch;
   if (!g) return;
   free_oneshot(g);
   for (void* p : {(void*)g->row_ptr, (void*)g->edges, (void*)g->post, (void*)g->col_of,
@@ -310,6 +311,7 @@ static int upload_graph(const snc_graph_view* v, Graph* g) {
 // (neuron, drive) entries sorted by neuron, each drive summed from 0.0f in
 // event order (cpu_backend.cpp:99).  ignore_sample maps every event to sample 0.
 void free_run(Run* r) {
+  const PoolBatch batch;
   if (!r) return;
   if (r->gexec) cudaGraphExecDestroy(r->gexec);
   if (r->outs) {

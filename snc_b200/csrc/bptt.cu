@@ -1331,6 +1331,7 @@ int snc_b200_bptt_set_resident(snc_b200_bptt* h, int32_t enable) {
 
 int snc_b200_bptt_release(snc_b200_bptt* h) {
   if (!h) return SNC_B200_OK;
+  const PoolBatch batch;
   for (void* p : {(void*)h->row_ptr, (void*)h->out_post, (void*)h->out_d, (void*)h->col_ptr,
                   (void*)h->in_pre, (void*)h->in_d, (void*)h->in_eidx, (void*)h->v, (void*)h->gv,
                   (void*)h->gcur, (void*)h->seg, (void*)h->part, (void*)h->ctl, (void*)h->err})

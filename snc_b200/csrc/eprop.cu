@@ -233,6 +233,7 @@ __global__ void k_elig_col(int B, int N, int S, int nc, int G, const int* cptr, 
 }
 
 static void free_session(snc_b200_eprop* s) {
+  const PoolBatch batch;
   for (void* p : {(void*)s->edges, (void*)s->bmat, (void*)s->internal_row, (void*)s->elig,
                   (void*)s->outs, (void*)s->delta, (void*)s->L, (void*)s->labels, (void*)s->fires})
     dev_free(p);
@@ -394,6 +395,7 @@ __global__ void k_apply_grad(int S, float lr, float w_max, int total_batch, cons
 static int run_batch(snc_b200_eprop* s, const snc_input_event* ev, size_t n_ev, int B,
                      const int32_t* steps, const int32_t* labels, int train, float* counts_out,
                      snc_run_stats* stats, float* grad = nullptr) {
+  const PoolBatch batch;
   const Graph* g = s->g;
   if (B < 1 || B > s->max_batch || !steps || (train && !labels)) {
     set_error("e-prop batch: bad sample count, steps or labels");

@@ -40,6 +40,13 @@ WaitCtl take_wait_ctl(bool consume);
 int pool_alloc(void** p, size_t n);
 int pool_alloc_host(void** p, size_t n);
 void pool_free(void* p);
+// What this thread releases in its scope is taken back at its end, with one wait.
+struct PoolBatch {
+  PoolBatch();
+  ~PoolBatch();
+  PoolBatch(const PoolBatch&) = delete;
+  PoolBatch& operator=(const PoolBatch&) = delete;
+};
 
 template <typename T>
 int dev_alloc(T** d, size_t n) {

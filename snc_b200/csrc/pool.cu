@@ -18,6 +18,7 @@
 #include <map>
 #include <mutex>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -129,10 +130,62 @@ bool wait_device(Pool& q, int dev) {
   return ok;
 }
 
+// Takes back blocks, after one wait for each of their devices: nothing that was
+// launched before this call may still use them.
+void give_back(const std::vector<void*>& ps) {
+  if (ps.empty()) return;
+  Pool& q = pool();
+  std::vector<std::pair<void*, Block>> bs;
+  {
+    std::lock_guard<std::mutex> lk(q.mu);
+    for (void* p : ps) {
+      auto it = q.live.find(p);
+      if (it != q.live.end()) bs.push_back(*it);
+    }
+  }
+  const RelaxedCapture relaxed;
+  int cur = 0;
+  const bool known = cudaGetDevice(&cur) == cudaSuccess;
+  std::map<int, bool> idle;  // by Block::dev
+  for (const auto& b : bs) {
+    const int dev = b.second.dev;
+    if (!known || idle.count(dev)) continue;
+    const bool sw = dev != kHost && cur != dev;
+    if (sw) cudaSetDevice(dev);
+    idle[dev] = wait_device(q, sw ? dev : cur);
+    if (sw) cudaSetDevice(cur);
+  }
+  std::lock_guard<std::mutex> lk(q.mu);
+  for (const auto& pb : bs) {
+    const Block& b = pb.second;
+    q.live.erase(pb.first);
+    size_t& kept = q.kept_bytes[b.dev];
+    if (idle[b.dev] && b.classed && kept + b.bytes <= keep_limit(b.dev)) {
+      q.kept[{b.dev, b.bytes}].push_back(pb.first);
+      kept += b.bytes;
+    } else {
+      raw_free(pb.first, b.dev);
+      cudaGetLastError();
+    }
+  }
+  if (q.live.empty()) {
+    for (auto& k : q.kept_bytes) trim(q, k.first);
+    for (auto& t : q.tokens) {
+      if (t.second.anchor) cudaFree(t.second.anchor);
+      if (t.second.spare) cudaFree(t.second.spare);
+      t.second = Token();
+    }
+  }
+}
+
+// Blocks that this thread releases within a PoolBatch.
+thread_local int later_depth = 0;
+thread_local std::vector<void*> later;
+
 int take(void** out, size_t n, int dev) {
   size_t c = size_class(n, dev);
   Pool& q = pool();
-  std::lock_guard<std::mutex> lk(q.mu);
+  std::unique_lock<std::mutex> lk(q.mu);
   auto& list = q.kept[{dev, c}];
   void* p = nullptr;
   if (!list.empty()) {
@@ -143,6 +196,9 @@ int take(void** out, size_t n, int dev) {
     cudaError_t e = raw_alloc(&p, c, dev);
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
+      lk.unlock();
+      give_back(std::exchange(later, {}));
+      lk.lock();
       trim(q, dev);
       c = n;  // what was asked for is what must fit
       e = raw_alloc(&p, c, dev);
@@ -171,40 +227,14 @@ int pool_alloc_host(void** p, size_t n) {
 
 void pool_free(void* p) {
   if (!p) return;
-  Pool& q = pool();
-  Block b;
-  {
-    std::lock_guard<std::mutex> lk(q.mu);
-    auto it = q.live.find(p);
-    if (it == q.live.end()) return;
-    b = it->second;
-  }
-  // nothing that was launched before this call may still use the block
-  const RelaxedCapture relaxed;
-  int cur = 0;
-  const bool known = cudaGetDevice(&cur) == cudaSuccess;
-  const bool sw = b.dev != kHost && known && cur != b.dev;
-  if (sw) cudaSetDevice(b.dev);
-  const bool idle = known && wait_device(q, sw ? b.dev : cur);
-  std::lock_guard<std::mutex> lk(q.mu);
-  q.live.erase(p);
-  size_t& kept = q.kept_bytes[b.dev];
-  if (idle && b.classed && kept + b.bytes <= keep_limit(b.dev)) {
-    q.kept[{b.dev, b.bytes}].push_back(p);
-    kept += b.bytes;
-  } else {
-    raw_free(p, b.dev);
-    cudaGetLastError();
-  }
-  if (q.live.empty()) {
-    for (auto& k : q.kept_bytes) trim(q, k.first);
-    for (auto& t : q.tokens) {
-      if (t.second.anchor) cudaFree(t.second.anchor);
-      if (t.second.spare) cudaFree(t.second.spare);
-      t.second = Token();
-    }
-  }
-  if (sw) cudaSetDevice(cur);
+  if (later_depth) later.push_back(p);
+  else give_back({p});
+}
+
+PoolBatch::PoolBatch() { ++later_depth; }
+
+PoolBatch::~PoolBatch() {
+  if (--later_depth == 0) give_back(std::exchange(later, {}));
 }
 
 }  // namespace sncb

@@ -647,6 +647,7 @@ void place_schedule(Inputs* in, void* dev) {
 // the legacy stream and waited for, the work block freed afterwards.
 int upload_inputs(const Graph* g, const snc_input_event* ev, size_t n_ev, int B,
                   const int32_t* steps, bool ignore_sample, Inputs* in) {
+  const PoolBatch batch;
   HostImage img;
   DevBuf keep, work;
   int rc = stage_inputs(g, ev, n_ev, B, steps, ignore_sample, in, &img, &keep, &work, nullptr, false);
@@ -750,6 +751,7 @@ __global__ void k_enc_write(EncArgs a) {
 
 int encode_inputs(const Graph* g, int enc, const float* features, int C, int B, const int32_t* steps,
                   float gain, float max_rate, float threshold, uint64_t seed, Inputs* in) {
+  const PoolBatch batch;
   if (enc < SNC_B200_ENCODER_DIRECT || enc > SNC_B200_ENCODER_LATENCY || C < 0 || B < 0 ||
       (B > 0 && !steps) || ((long long)B * C > 0 && !features)) {
     set_error("encode: bad arguments");

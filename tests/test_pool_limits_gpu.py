@@ -64,3 +64,20 @@ train(s); E.destroy(s)
 dg.release()
 assert a - free() <= 16 * MiB
 """)
+
+
+def test_a_minibatch_that_outgrows_its_scratch():
+    """The scratch that a longer minibatch replaces makes room for the new one
+    before the call ends."""
+    _run("""
+s = session(1)
+n = 2 * 305 * 4                          # bytes of surrogate history a step
+long = 1200 * MiB // n
+def run(T):
+    ev = W.random_events(4, g, 2, 4)[0]
+    s.run_batch(ev, np.full(2, T, np.int32), np.zeros(2, np.int32), train=True)
+run(long * 2 // 3)                       # 800 MiB of history
+b = leave(600)                           # the 1200 fit only in their place
+run(long)
+assert np.count_nonzero(s.eligibility(2))
+""")
