@@ -28,10 +28,10 @@
 // shared memory and all warps are co-resident (up to 32 an SM, degrees up to
 // 256); k_bptt_forward / k_bptt_backward take everything else (the smoothed
 // variant, larger graphs) and give the same bits.  Measured: 4096 recurrent
-// neurons, fan-in 64, 64 samples, 256 steps: forward 1.05 ms, backward 3.5 ms
+// neurons, fan-in 64, 64 samples, 256 steps: forward 1.02 ms, backward 3.21 ms
 // (1.9 and 6.8 with the general form, a warp per neuron walking all spike words
 // and gradients through shuffles, its weight gradients before the barrier);
-// 784-512-512 at 128 samples, 100 steps: 0.59 and 1.71 ms (1.0 and 3.57).
+// 784-512-512 at 128 samples, 100 steps: 0.59 and 1.68 ms (1.0 and 3.57).
 // What is left is latency: a grid barrier and two L2 trips a step, and in the
 // backward 458 KB of gradients an SM gathers from L2 each step (7000 cycles at
 // 64 B a cycle, of 27000).
@@ -534,11 +534,12 @@ __global__ void __launch_bounds__(kBpThreads, kBpMinBlocks<KB>) k_bptt_backward(
 // between the arrival at a step's barrier and the wait for it.  G lies in a
 // ring whose rows start on VB floats, read as VB-wide vectors; lanes beyond the
 // batch read the next row (there is room behind the last) and drop what they
-// get.  Rows of steps beyond T are zero.  Edge offsets of a step are computed once per edge and passed through
-// shared memory.  The last steps, as many as the largest delay, stage the edges
-// anew with weight 0 for those that reach beyond T (an infinite weight times a
-// zero gradient would be NaN), so the gather needs no check; a check per offset
-// there took 1.7 % of the backward of 4096 neurons, staging takes nothing.
+// get.  Rows of steps beyond T are zero.  Edge offsets of a step are computed
+// once per edge and passed through shared memory.  The last steps, as many as
+// the largest delay, stage the edges anew with weight 0 for those that reach
+// beyond T (an infinite weight times a zero gradient would be NaN), about 2 us a
+// step, so the gather needs no check (one per offset took 1.7 % of the backward
+// of 4096 neurons, 256 steps).
 //
 // Items go round the CTAs (item i to CTA i mod grid), so that neurons without
 // synapses in one direction share an SM with others; where every run of 32

@@ -479,10 +479,10 @@ __device__ __forceinline__ void stage_row(const int* __restrict__ sptr, int j, i
 // 2600, list and the copy of the segment starts 1400 and 900 (L2), a warp's
 // segments 2300, its first edges 600 (L2), 7 groups of 32 events a warp 7500 --
 // eight warps a scheduler, two thirds of a group shared-memory passes over
-// random cells (tag, ring).  7.9 us a step, 17.2 with events staged 1024 at a
+// random cells (tag, ring).  7.5 us a step, 17.2 with events staged 1024 at a
 // time by a search per event and ordered through cell bitmaps and a hash table;
-// ATOMIC 4.1 us, 6.0 with the rows of a warp's list fetched one after another;
-// a 1050-neuron net with 90 short rows a step 4.3 us, 5.2 before.  Clusters of
+// ATOMIC 4.0 us, 6.0 with the rows of a warp's list fetched one after another;
+// a 1050-neuron net with 90 short rows a step 4.2 us, 5.2 before.  Clusters of
 // four: 5.8 us for up to 33 samples.  Slower: 16 ranges and warps (too few in
 // flight), owners that add one row's segment at a time without a conflict check
 // (130 cycles a row for the chain), match.any for the conflicts (100 cycles a
